@@ -991,6 +991,33 @@ static int persistent_grid(const void* kernel, int threads, size_t smem, long lo
   return (int)std::min<long long>(*cache, planes);
 }
 
+// Default schedules of a group of n droplets of size N. fused_rhs: the persistent grid (within 3 %
+// of the best chunk at every group size measured). fused_div and fused_correct: chunks of z-planes,
+// long enough to amortise the stencils' two halo planes and the ring's first copies, but short
+// enough that one wave of CTAs covers every SM: the planes are cut into as many chunks as one wave
+// holds (3 or 2 CTAs per SM), at most 40 (fused_div) or 20 (fused_correct) planes each. Measured, us
+// per launch: one 64^3 droplet (8 tiles; 2 planes per chunk instead of a single chunk of 64) 82 ->
+// 15 and 64 -> 11; 2 x 96^3 86 -> 35 and 75 -> 29; 12 x 128^3 (the caps; longer chunks leave a partial
+// last wave, shorter ones re-read halos: 8 planes 336 / 315, 64 planes 325 / 335) 325 -> 309 and
+// 335 -> 310; 2 x 256^3 378 -> 376 and 430 -> 409.
+void fused_default_zc(int N, int n, int zc[3]) {
+  int dev = 0, sms = 0;
+  check(cudaGetDevice(&dev), "fused: device");
+  check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "fused: SM count");
+  auto planes = [&](int per_sm, int th, int most) {
+    const long long tiles = (long long)n * (N / TX) * (N / th);
+    const long long wave = std::max<long long>(1, (long long)sms * per_sm / tiles);  // chunks of one wave
+    const int w = (int)std::min<long long>(wave, N);
+    const int z = std::min(most, (N + w - 1) / w);
+    const int chunks = (N + z - 1) / z;
+    if ((long long)chunks * n > 65535) return N;  // the grid's limit: very many small droplets
+    return (N + chunks - 1) / chunks;             // equal chunks
+  };
+  zc[0] = 0;
+  zc[1] = planes(3, TYD, 40);
+  zc[2] = planes(2, TY, 20);
+}
+
 template <class K>
 static void launch_sweep(K chunked, K persistent, const Group<float>& g, int par, int zc, int th, int threads, size_t smem,
                          int* cache, cudaStream_t st, const char* what) {

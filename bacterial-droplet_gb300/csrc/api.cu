@@ -228,7 +228,6 @@ Phys<T> make_phys(const ttsh_input& in, const ttsh_ext& ext) {
   p.h = (T)h;
   p.dt = (T)in.dt0;
   p.inv_dt = (T)(1.0 / in.dt0);
-  p.dt_d = in.dt0;
   p.mu = (T)in.mu; p.cA = (T)in.cA; p.alpha = (T)in.alpha; p.beta = (T)in.beta; p.eta = (T)in.eta;
   p.La2 = (T)(in.La * in.La);
   p.kappa = (T)in.kappa; p.lambda0 = (T)in.lambda0;
@@ -239,6 +238,7 @@ Phys<T> make_phys(const ttsh_input& in, const ttsh_ext& ext) {
   p.cl23 = (T)(2.0 / (3 * h * h));
   p.cl143 = (T)(14.0 / (3 * h * h));
   p.clz = (T)(1.0 / (h * h));
+  separable_constants(p, h, in.dt0, in.kPhi, in.La, in.mu, in.gamma, in.eta);
   const double n3 = (double)in.Nx * in.Nx * in.Nx;
   p.invN3 = (T)(1.0 / n3);
   return p;
@@ -302,6 +302,7 @@ void build_engine(ttsh_sim* s, Engine<T>& E) {
     t.Ct = reinterpret_cast<T*>(d + off); CK(cudaMemcpy(d + off, Ct.data(), N * sizeof(T), cudaMemcpyHostToDevice));
     tab[N] = t;
     fft_prepare<T>(N);
+    if (sizeof(T) == 8) plain64_prepare(N);
     if (fftreg_has<T>(N)) fftreg_twiddles<T>(N);
   }
   // per-instance arenas

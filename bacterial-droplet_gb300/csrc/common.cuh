@@ -23,8 +23,22 @@ struct Phys {
   T cl12, cl23, cl143;  // 1/(12h^2), 2/(3h^2), 14/(3h^2)
   T clz;           // 1/h^2 (the fused form's shift-invariant Laplacian)
   T invN3;         // 1/N^3 (FP32 path); FP64 path divides by (double)N^3 as getStream mode 2
-  double dt_d;     // dt in FP64 (divisor of getStream mode 0 in the FP64 path)
+  // constants of the FP64 form's separable stencils, whose sums have integer weights: 1/(72 h) of D,
+  // the same over dt, and 1/(12 h^2) of L times kPhi, La^2, mu, gamma, eta
+  T kd, kdiv, kPhi12, La212, mu12, gamma12, eta12;
 };
+
+template <class T>
+inline void separable_constants(Phys<T>& p, double h, double dt, double kPhi, double La, double mu, double gamma, double eta) {
+  const double l12 = 12 * h * h;
+  p.kd = (T)(1.0 / (72 * h));
+  p.kdiv = (T)(1.0 / (72 * h * dt));
+  p.kPhi12 = (T)(kPhi / l12);
+  p.La212 = (T)(La * La / l12);
+  p.mu12 = (T)(mu / l12);
+  p.gamma12 = (T)(gamma / l12);
+  p.eta12 = (T)(eta / l12);
+}
 
 // Per-droplet device descriptor. Field arrays are unpadded N^3, x fastest.
 // Ping-pong pairs are indexed by the step parity `par`: the step reads

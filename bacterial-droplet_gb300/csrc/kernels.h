@@ -31,11 +31,22 @@ struct Group {
   int* d_err = nullptr;  // set to 1 by a kernel whose bounded wait for its input ran out
 };
 
-// Plain form (one thread per site, reference arithmetic order), plain.cu.
+// Plain form (global intermediates): FP32 one thread per site in the reference's arithmetic order
+// (plain.cu), FP64 separable stencils on tiles of one z-plane (plain64.cu).
 template <class T> void launch_stage1(const Group<T>& g, int par, cudaStream_t st);
 template <class T> void launch_stage2(const Group<T>& g, int par, cudaStream_t st);
 template <class T> void launch_div(const Group<T>& g, int par, cudaStream_t st);
 template <class T> void launch_correct(const Group<T>& g, int par, cudaStream_t st);
+// Sets the FP64 kernels' dynamic shared-memory limits for size N (call before capture).
+void plain64_prepare(int N);
+template <> void launch_stage1<float>(const Group<float>&, int, cudaStream_t);
+template <> void launch_stage2<float>(const Group<float>&, int, cudaStream_t);
+template <> void launch_div<float>(const Group<float>&, int, cudaStream_t);
+template <> void launch_correct<float>(const Group<float>&, int, cudaStream_t);
+template <> void launch_stage1<double>(const Group<double>&, int, cudaStream_t);
+template <> void launch_stage2<double>(const Group<double>&, int, cudaStream_t);
+template <> void launch_div<double>(const Group<double>&, int, cudaStream_t);
+template <> void launch_correct<double>(const Group<double>&, int, cudaStream_t);
 // FP64 diagnostics: per-instance partials into d_inst[i].red (nblocks_out per instance).
 template <class T> int launch_stats(const Group<T>& g, int par, cudaStream_t st, bool full = true);
 int stats_partials_per_instance(int N);

@@ -25,7 +25,7 @@
 //   * Every later call only enqueues work on the caller's stream: the tables and the droplet
 //     descriptor travel as the parameter of a small set-up kernel (copied at launch), not through
 //     host memory that a copy would have to wait for or outlive.
-// The step kernels are the plain-form kernels of plain.cu and fft.cu, unchanged.
+// The step kernels are the plain-form kernels of plain64.cu and fft.cu, unchanged.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -134,6 +134,7 @@ extern "C" int ttsh_step_noalloc(const ttsh_input* in, const ttsh_ext* ext, int 
       std::lock_guard<std::mutex> lk(g_mu);
       if (!g_prepared[dev][N]) {
         fft_prepare<double>(N);
+        plain64_prepare(N);
         if (fftreg_has<double>(N)) fftreg_twiddles<double>(N);  // the register FFT's constant table
         // the table copy runs on the legacy stream: let it land before kernels on any stream read it
         const cudaError_t es = cudaDeviceSynchronize();
@@ -185,12 +186,13 @@ extern "C" int ttsh_step_noalloc(const ttsh_input* in, const ttsh_ext* ext, int 
     while (m % 5 == 0) { I.radix[ns++] = 5; m /= 5; }
     I.nstages = ns;
     Phys<double>& p = I.ph;
-    p.h = h; p.dt = in->dt0; p.inv_dt = 1.0 / in->dt0; p.dt_d = in->dt0;
+    p.h = h; p.dt = in->dt0; p.inv_dt = 1.0 / in->dt0;
     p.mu = in->mu; p.cA = in->cA; p.alpha = in->alpha; p.beta = in->beta; p.eta = in->eta;
     p.La2 = in->La * in->La; p.kappa = in->kappa; p.lambda0 = in->lambda0; p.aPhi2 = in->aPhi * 2;
     p.kPhi = in->kPhi; p.gamma = in->gamma; p.A = in->A; p.zeta = ext->zeta;
     p.c2h = 1.0 / (2.0 * h); p.cl12 = 1.0 / (12 * h * h); p.cl23 = 2.0 / (3 * h * h); p.cl143 = 14.0 / (3 * h * h);
     p.invN3 = 1.0 / ((double)N * N * N);
+    separable_constants(p, h, in->dt0, in->kPhi, in->La, in->mu, in->gamma, in->eta);
     I.phi[0] = phi; I.phi[1] = phi_new;
     for (int b = 0; b < 3; ++b) {
       I.P[b] = P + b * n;

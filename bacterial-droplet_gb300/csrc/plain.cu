@@ -1,7 +1,7 @@
-// plain.cu — the plain form of the TTSH3D step: one thread per lattice site, the
-// reference's stencils evaluated in its arithmetic order, global intermediates.
-// It is the FP64 form of the step (and an FP32 form for cross-checks); the fused
-// FP32 kernels in fused.cu replace stage1/stage2/div for speed.
+// plain.cu — the FP32 plain form of the TTSH3D step: one thread per lattice site, the
+// reference's stencils evaluated in its arithmetic order, global intermediates (sizes that are no
+// multiple of 32, and cross-checks). plain64.cu is the FP64 form; the fused FP32 kernels in fused.cu
+// replace stage1/stage2/div for speed. The diagnostics serve every form.
 //
 //   stage1  <- getTempVari_1 + getTempVari_2 (TTSH3D.cu:537-605): mu_0, mu_b, sigma_ab
 //   stage2  <- getDtF + getVStar + phi update of getVNew (:608-632, :471-491, :515)
@@ -121,13 +121,6 @@ __global__ void __launch_bounds__(BX* BY) k_stage2(const InstDev<T>* __restrict_
 }
 
 template <class T>
-__device__ __forceinline__ T divide_dt(T a, const Phys<T>& p);
-template <>
-__device__ __forceinline__ double divide_dt<double>(double a, const Phys<double>& p) { return a / p.dt_d; }
-template <>
-__device__ __forceinline__ float divide_dt<float>(float a, const Phys<float>& p) { return a * p.inv_dt; }
-
-template <class T>
 __global__ void __launch_bounds__(BX* BY) k_div(const InstDev<T>* __restrict__ insts, int par) {
   const int N = insts[0].N;
   const InstDev<T>& I = insts[blockIdx.z / N];
@@ -152,7 +145,7 @@ __global__ void __launch_bounds__(BX* BY) k_div(const InstDev<T>* __restrict__ i
       b = st_dy<T>(s.acc<T>(cur[1]), p.c2h);
       c = st_dz<T>(s.acc<T>(cur[2]), p.c2h);
     }
-    d[f] = divide_dt<T>(a + b + c, p);  // getStream mode 0 (:666-668)
+    d[f] = (a + b + c) * p.inv_dt;  // getStream mode 0 (:666-668)
   }
   typename CxT<T>::type w;
   w.x = d[0];
@@ -315,24 +308,24 @@ __global__ void __launch_bounds__(STATS_THREADS) k_stats(const InstDev<T>* __res
 
 int stats_partials_per_instance(int) { return STATS_BLOCKS; }
 
-template <class T>
-void launch_stage1(const Group<T>& g, int par, cudaStream_t st) {
-  k_stage1<T><<<site_grid(g.N, g.n), dim3(BX, BY), 0, st>>>(g.d_inst, par);
+template <>
+void launch_stage1<float>(const Group<float>& g, int par, cudaStream_t st) {
+  k_stage1<float><<<site_grid(g.N, g.n), dim3(BX, BY), 0, st>>>(g.d_inst, par);
   check_launch("stage1");
 }
-template <class T>
-void launch_stage2(const Group<T>& g, int par, cudaStream_t st) {
-  k_stage2<T><<<site_grid(g.N, g.n), dim3(BX, BY), 0, st>>>(g.d_inst, par);
+template <>
+void launch_stage2<float>(const Group<float>& g, int par, cudaStream_t st) {
+  k_stage2<float><<<site_grid(g.N, g.n), dim3(BX, BY), 0, st>>>(g.d_inst, par);
   check_launch("stage2");
 }
-template <class T>
-void launch_div(const Group<T>& g, int par, cudaStream_t st) {
-  k_div<T><<<site_grid(g.N, g.n), dim3(BX, BY), 0, st>>>(g.d_inst, par);
+template <>
+void launch_div<float>(const Group<float>& g, int par, cudaStream_t st) {
+  k_div<float><<<site_grid(g.N, g.n), dim3(BX, BY), 0, st>>>(g.d_inst, par);
   check_launch("div");
 }
-template <class T>
-void launch_correct(const Group<T>& g, int par, cudaStream_t st) {
-  k_correct<T><<<site_grid(g.N, g.n), dim3(BX, BY), 0, st>>>(g.d_inst, par);
+template <>
+void launch_correct<float>(const Group<float>& g, int par, cudaStream_t st) {
+  k_correct<float><<<site_grid(g.N, g.n), dim3(BX, BY), 0, st>>>(g.d_inst, par);
   check_launch("correct");
 }
 template <class T>
@@ -343,14 +336,7 @@ int launch_stats(const Group<T>& g, int par, cudaStream_t st, bool full) {
   return STATS_BLOCKS;
 }
 
-#define INST(T)                                                          \
-  template void launch_stage1<T>(const Group<T>&, int, cudaStream_t);   \
-  template void launch_stage2<T>(const Group<T>&, int, cudaStream_t);   \
-  template void launch_div<T>(const Group<T>&, int, cudaStream_t);      \
-  template void launch_correct<T>(const Group<T>&, int, cudaStream_t);  \
-  template int launch_stats<T>(const Group<T>&, int, cudaStream_t, bool);
-INST(float)
-INST(double)
-#undef INST
+template int launch_stats<float>(const Group<float>&, int, cudaStream_t, bool);
+template int launch_stats<double>(const Group<double>&, int, cudaStream_t, bool);
 
 }  // namespace ttsh

@@ -507,8 +507,8 @@ def main():
             ms64 = replicas.max_over_ranks(a.elapsed_time(b), device="cuda")
         v64 = 256 ** 3 * world * k64 / (ms64 / 1e3) / 1e6
         fp64 = {"value": v64, "unit": UNIT, "ms_per_step": ms64 / k64, "steps": k64, "warmup": 3,
-                "workload": "1 x 256^3 (R=64, xi=2, seed 1, zeta=0.02), FP64 plain form (one droplet per launch, "
-                            "the reference's arithmetic order), same GPU and run",
+                "workload": "1 x 256^3 (R=64, xi=2, seed 1, zeta=0.02), FP64 plain form (one droplet per launch), "
+                            "same GPU and run",
                 "ratio_fp32_batched_over_fp64_plain": value / v64}
 
     cpu = None

@@ -63,7 +63,8 @@ typedef struct ttsh_ext {
   int form;        /* TTSH_FORM_AUTO, TTSH_FORM_PLAIN or TTSH_FORM_FUSED (same for all droplets) */
 } ttsh_ext;
 #define TTSH_FORM_AUTO 0   /* fused kernels where supported (FP32, N a multiple of 32), else plain */
-#define TTSH_FORM_PLAIN 1  /* one thread per site, the reference's arithmetic order (FP64 or FP32) */
+#define TTSH_FORM_PLAIN 1  /* every intermediate in an array of its own (FP64 or FP32; FP32 in the reference's
+                              arithmetic order, FP64 with its stencils summed separably) */
 #define TTSH_FORM_FUSED 2  /* fused FP32 kernels; TTSH_E_UNSUPPORTED where they do not apply */
 
 typedef struct ttsh_stats {

@@ -67,20 +67,20 @@ const char* kNames[K_NCLASS] = {"stage1", "stage2", "div", "fft_x_fwd", "fft_y_f
                                 "fft_x_inv", "correct", "fused_rhs", "fused_div", "fused_correct",
                                 "fft_xy_fwd", "fft_yx_inv"};
 
-// The Poisson solve of a group: x+y per plane, z, y+x per plane (fft_kind 2 with a register
-// kernel for the size), else one launch per axis pass. `run(class, launch)` wraps each launch.
+// The Poisson solve of a group: x+y per plane, z, y+x per plane (fft_kind 2), else one launch per
+// axis pass. `run(class, launch)` wraps each launch.
 template <class T, class R>
 void enqueue_fft(const Group<T>& g, cudaStream_t st, R&& run) {
-  if (g.fft_kind == 2 && fftreg_has<T>(g.N)) {
-    run(K_FFT_XY, [&] { fftreg_plane_launch<T>(g, 0, st); });
+  if (g.fft_kind == 2) {
+    run(K_FFT_XY, [&] { launch_fft_plane<T>(g, 0, st); });
     run(K_FFT2, [&] { launch_fft_pass<T>(g, 2, st); });
-    run(K_FFT_YX, [&] { fftreg_plane_launch<T>(g, 1, st); });
+    run(K_FFT_YX, [&] { launch_fft_plane<T>(g, 1, st); });
   } else {
     for (int pass = 0; pass < 5; ++pass) run(K_FFT0 + pass, [&] { launch_fft_pass<T>(g, pass, st); });
   }
 }
 template <class T>
-int fft_launches(const Group<T>& g) { return (g.fft_kind == 2 && fftreg_has<T>(g.N)) ? 3 : 5; }
+int fft_launches(const Group<T>& g) { return g.fft_kind == 2 ? 3 : 5; }
 
 struct Prof {
   cudaStream_t st;
@@ -330,6 +330,7 @@ void build_engine(ttsh_sim* s, Engine<T>& E) {
     std::vector<int> r = radix_plan(N);
     I.nstages = (int)r.size();
     for (size_t k = 0; k < r.size(); ++k) I.radix[k] = r[k];
+    fft_steps<T>(N, r, I.step, &I.nsteps);
     I.ph = make_phys<T>(ih.in, ih.ext);
     size_t off = 0;
     auto take = [&]() { T* p = reinterpret_cast<T*>(d + off); off += fb; return p; };
@@ -395,6 +396,7 @@ void build_engine(ttsh_sim* s, Engine<T>& E) {
     G.fft_kind = (fk && std::string(fk) == "stockham") ? 1 : ((fk && std::string(fk) == "separate") ? 0 : 2);
     G.n = (int)E.members[g].size();
     G.N = s->inst[E.members[g][0]].N;
+    G.fft_nsteps = E.h[E.members[g][0]].nsteps;
     G.d_err = s->d_err;
     if (s->fused) fused_default_zc(G.N, G.n, G.zc);
     // FP32, on request (TTSH_ZTMA=1): the z pass with its input staged by the tensor memory
@@ -568,6 +570,8 @@ void set_radix(ttsh_sim* s, Engine<T>& E, size_t gi, const std::vector<int>& r) 
   for (int i : E.members[gi]) {
     E.h[i].nstages = (int)r.size();
     for (size_t k = 0; k < r.size(); ++k) E.h[i].radix[k] = r[k];
+    fft_steps<T>(E.h[i].N, r, E.h[i].step, &E.h[i].nsteps);
+    E.groups[gi].fft_nsteps = E.h[i].nsteps;
   }
   upload_group(s, E, gi);
 }
@@ -690,10 +694,8 @@ void tune_group(ttsh_sim* s, Engine<T>& E, size_t gi, ttsh_tuning* out) {
     struct Cand { int kind, lb; std::vector<int> radix; };
     std::vector<Cand> cands;
     const std::vector<std::vector<int>> orders = radix_orders(G.N);
-    if (fftreg_has<T>(G.N)) {
-      cands.push_back({2, 0, orders[0]});
-      cands.push_back({0, 0, orders[0]});
-    }
+    cands.push_back({2, 0, orders[0]});
+    cands.push_back({0, 0, orders[0]});
     for (int lb : fft_lb_candidates<T>(G.N))
       for (const auto& o : orders) cands.push_back({1, lb, o});
     double best = 1e30;

@@ -47,7 +47,9 @@ template <class T>
 struct InstDev {
   typedef typename CxT<T>::type C;
   int N, stale, k2mode, nstages;
-  int radix[16];
+  int radix[16];      // the radix plan (factors 2 .. 5) as a tuning states it
+  int nsteps;         // the steps the FFT of fft.cu takes for it (fft_steps), radices 2 .. 16
+  int step[16];
   Phys<T> ph;
   T* phi[2];
   T* P[3];

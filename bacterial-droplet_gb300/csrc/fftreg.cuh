@@ -5,11 +5,12 @@
 //   X[k1 + N1*k2] = DFT_N2 over n2 of w_N^(n2*k1) * Y[k1][n2]    (after one shared-memory transpose)
 // and the inverse runs the same steps backwards. Each thread keeps its N1 (or N2) values in
 // registers; small DFTs are expanded at compile time by mixed-radix decimation in time
-// (radix 4, 2, 3, 5), with twiddles read from the FP64-built table exp(-2 pi i k / N).
+// (radix 4, 2, and the 3- and 5-point ones of dft.cuh), with twiddles read from the FP64-built table exp(-2 pi i k / N).
 // The z pass goes forward, applies the Poisson multiplier and goes back without leaving the
 // CTA: two shared-memory transposes for the whole forward-divide-inverse sequence.
 #pragma once
 #include "common.cuh"
+#include "dft.cuh"
 
 namespace ttsh {
 namespace fftreg {
@@ -84,6 +85,16 @@ struct Dft {
       v[2] = csub(a, c);
       v[1] = cadd(b, dd);
       v[3] = csub(b, dd);
+    } else if constexpr ((L == 3 || L == 5) && sizeof(v->x) == 8) {
+      dft::Dft<L>::run(v);
+      if (INV) {  // the inverse transform's output k is the forward one's -k
+#pragma unroll
+        for (int k = 1; 2 * k < L; ++k) {
+          const C t = v[k];
+          v[k] = v[L - k];
+          v[L - k] = t;
+        }
+      }
     } else if constexpr (L == 3 || L == 5) {
       C o[L];
 #pragma unroll
@@ -117,39 +128,54 @@ struct Dft {
   }
 };
 
-// -F / k^2 of getStream mode 1 (:672-683) with k2 from initPoissonSolver (:1088-1124).
-__device__ __forceinline__ double2 poisson_mul(double2 v, const InstDev<double>& I, int x, int y, int z) {
-  double k2;
-  if (I.k2mode == 0) {
-    const double kx = I.kval[x], ky = I.kval[y], kz = I.kval[z];
-    // the host's kx*kx + ky*ky + kz*kz, without contraction
-    k2 = __dadd_rn(__dadd_rn(__dmul_rn(kx, kx), __dmul_rn(ky, ky)), __dmul_rn(kz, kz));
-    if ((x | y | z) == 0) k2 = 1;  // k2[0] = 1 (:1120)
-  } else {
-    const double Kx = I.St[x] * I.Ct[y] * I.Ct[z], Ky = I.Ct[x] * I.St[y] * I.Ct[z], Kz = I.Ct[x] * I.Ct[y] * I.St[z];
-    k2 = Kx * Kx + Ky * Ky + Kz * Kz;
-    if (k2 < 1e-8 / ((double)I.ph.h * (double)I.ph.h)) return make_double2(0.0, 0.0);
+// -F / k^2 of getStream mode 1 (:672-683) with k2 from initPoissonSolver (:1088-1124), along the z
+// line at (x, y). In FP64 k2 is the host's kx*kx + ky*ky + kz*kz bit for bit (rounded squares, no
+// contraction); the spectrum is multiplied by one reciprocal instead of divided twice (an FP64
+// division takes about ten operations).
+template <class T>
+struct Poisson {
+  T a, b, c;
+  bool line0;  // x = y = 0
+  __device__ __forceinline__ Poisson(const InstDev<T>& I, int x, int y) {
+    line0 = (x | y) == 0;
+    if (I.k2mode == 0) {
+      a = sum(I.k2t[x], I.k2t[y]);
+      b = c = T(0);
+    } else {
+      a = I.St[x] * I.Ct[y];
+      b = I.Ct[x] * I.St[y];
+      c = I.Ct[x] * I.Ct[y];
+    }
   }
-  return make_double2(-v.x / k2, -v.y / k2);
-}
-__device__ __forceinline__ float2 poisson_mul(float2 v, const InstDev<float>& I, int x, int y, int z) {
-  float k2;
-  if (I.k2mode == 0) {
-    k2 = I.k2t[x] + I.k2t[y] + I.k2t[z];
-    if ((x | y | z) == 0) k2 = 1.f;
-  } else {
-    const float Kx = I.St[x] * I.Ct[y] * I.Ct[z], Ky = I.Ct[x] * I.St[y] * I.Ct[z], Kz = I.Ct[x] * I.Ct[y] * I.St[z];
-    k2 = Kx * Kx + Ky * Ky + Kz * Kz;
-    if (k2 < 1e-8f / (I.ph.h * I.ph.h)) return make_float2(0.f, 0.f);
+  static __device__ __forceinline__ double sum(double u, double v) { return __dadd_rn(u, v); }
+  static __device__ __forceinline__ float sum(float u, float v) { return __fadd_rn(u, v); }
+  static __device__ __forceinline__ double reciprocal(double v) { return 1.0 / v; }
+  static __device__ __forceinline__ float reciprocal(float v) { return __frcp_rn(v); }  // the value of 1.f / v
+  template <class C>
+  __device__ __forceinline__ C operator()(C v, const InstDev<T>& I, int z) const {
+    T k2;
+    C o;
+    if (I.k2mode == 0) {
+      k2 = sum(a, I.k2t[z]);
+      if (line0 && z == 0) k2 = T(1);  // k2[0] = 1 (:1120)
+    } else {
+      const T ct = I.Ct[z], Kx = a * ct, Ky = b * ct, Kz = c * I.St[z];
+      k2 = Kx * Kx + Ky * Ky + Kz * Kz;
+      if (k2 < T(1e-8) / (I.ph.h * I.ph.h)) {
+        o.x = o.y = T(0);
+        return o;
+      }
+    }
+    const T f = -reciprocal(k2);
+    o.x = v.x * f;
+    o.y = v.y * f;
+    return o;
   }
-  // the correctly rounded reciprocal: the value of -1.f / k2 without a full division routine
-  const float f = -__frcp_rn(k2);
-  return make_float2(v.x * f, v.y * f);
-}
+};
 
+// getStream mode 2 (:684-690): times 1/N^3 (exact where N is a power of two)
 __device__ __forceinline__ double2 scale_n3(double2 v, const InstDev<double>& I) {
-  const double n3 = (double)(I.N * I.N * I.N);
-  return make_double2(v.x / n3, v.y / n3);
+  return make_double2(v.x * I.ph.invN3, v.y * I.ph.invN3);
 }
 __device__ __forceinline__ float2 scale_n3(float2 v, const InstDev<float>& I) {
   return make_float2(v.x * I.ph.invN3, v.y * I.ph.invN3);

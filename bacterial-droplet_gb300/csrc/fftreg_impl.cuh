@@ -165,6 +165,7 @@ __device__ __forceinline__ void fft_lines(const InstDev<T>& I, int g, typename C
     for (int k1 = 0; k1 < N1; ++k1) S[sidx(k1, j)] = (k1 > 0 && j > 0) ? cmul(v[k1], tw4<C, false, N, TW4C>(tab, j * k1)) : v[k1];
     __syncthreads();
     after();
+    const Poisson<T> pm(I, xl, yl);  // used by the z pass
 #pragma unroll
     for (int o = 0; o < OW; ++o) {
       const int k1 = j + N2 * o;
@@ -175,7 +176,7 @@ __device__ __forceinline__ void fft_lines(const InstDev<T>& I, int g, typename C
       if constexpr (PASS == 2) {
         // spectrum element z = k1 + N1*k2 of the line (x = xl, y = yl): multiply, go back
 #pragma unroll
-        for (int k2 = 0; k2 < N2; ++k2) u[k2] = poisson_mul(u[k2], I, xl, yl, k1 + N1 * k2);
+        for (int k2 = 0; k2 < N2; ++k2) u[k2] = pm(u[k2], I, k1 + N1 * k2);
         Dft<C, N2, true, N>::run(u, tab, N1);
 #pragma unroll
         for (int n2 = 0; n2 < N2; ++n2) S[sidx(k1, n2)] = (n2 > 0 && k1 > 0) ? cmul(u[n2], tw4<C, true, N, TW4C>(tab, n2 * k1)) : u[n2];

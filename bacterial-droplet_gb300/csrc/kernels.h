@@ -14,9 +14,10 @@ struct Group {
   InstDev<T>* d_inst;  // device array [n]
   int n;               // instances in the group
   int N;
-  int fft_kind = 0;    // register-resident FFT kernels where the size has them: 0 one launch per
-                       // axis pass, 2 x and y of a plane in one launch; 1: Stockham only
-  int fft_lb = 0;      // Stockham lines per CTA (0: the largest power of two that fits)
+  int fft_kind = 0;    // register-resident FFT kernels where the size has them, else Stockham: 0 one
+                       // launch per axis pass, 2 x and y of a plane in one launch; 1: Stockham only
+  int fft_lb = 0;      // Stockham lines per CTA (0: chosen by size, default_lb of fft.cu)
+  int fft_nsteps = 0;  // InstDev::nsteps of the group (0: not known, taken as three or more)
   int zc[3] = {0, 0, 0};     // z-planes per CTA of fused_rhs, fused_div, fused_correct
                              // (fused_default_zc); 0: the persistent grid (equal shares of the
                              // group's sites per CTA)
@@ -54,10 +55,17 @@ int stats_partials_per_instance(int N);
 // Poisson solve by FFT (fft.cu): W <- (inverse FFT of -FFT(W)/k^2) / N^3.
 // pass 0: forward x; 1: forward y; 2: forward z, divide, inverse z; 3: inverse y; 4: inverse x + scale.
 template <class T> void launch_fft_pass(const Group<T>& g, int pass, cudaStream_t st);
-template <class T> size_t fft_smem_bytes(int N, int pass);
+// Forward x + y (dir 0) or inverse y + x (dir 1) of every z-plane in one launch (fft_kind 2): the
+// register kernel of the size, else the one for any size.
+template <class T> void launch_fft_plane(const Group<T>& g, int dir, cudaStream_t st);
+// The steps the any-size FFT takes for a radix plan (product N, factors 2 .. 5, at most 16). FP32: its
+// stages, two at a time where a kernel has the pair. FP64: the best radices up to 16 for N when the
+// plan is the default order (4, 2, 3, 5) or its reverse, else consecutive factors of the plan merged.
+template <class T>
+void fft_steps(int N, const std::vector<int>& plan, int* step, int* nsteps);
 // Sets the dynamic shared-memory limits of the FFT kernels for size N (call before capture).
 template <class T> void fft_prepare(int N);
-// Stockham lines per CTA: the candidates for size N (largest first) and the one a group uses.
+// Stockham lines per CTA: the explicit candidates for size N (largest first) and the one a group uses.
 template <class T> std::vector<int> fft_lb_candidates(int N);
 template <class T> int fft_lines(const Group<T>& g);
 // Register-resident FFT passes (fftreg_*.cu): false when the size has none (Stockham is used).
@@ -67,8 +75,7 @@ template <class T> void fftreg_prepare(int N);
 // kernels read it; call once per device and size before they run; allocates nothing).
 template <class T> void fftreg_twiddles(int N);
 template <class T> bool fftreg_has(int N);
-// Forward x + y (dir 0) or inverse y + x (dir 1) of every z-plane, one CTA per plane (fft_kind 2):
-// false when the group does not use it.
+// The register kernel of launch_fft_plane: false when the size has none or the group does not use it.
 template <class T> bool fftreg_plane_launch(const Group<T>& g, int dir, cudaStream_t st);
 // The staged z pass of size N (FP32): builds the descriptors of the complex fields W[i] in a new
 // device array (*d_maps, caller frees) and returns the persistent grid; 0 when N has none.

@@ -33,6 +33,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <vector>
 
 #include "../../include/ttsh.h"
 #include "common.cuh"
@@ -179,12 +180,13 @@ extern "C" int ttsh_step_noalloc(const ttsh_input* in, const ttsh_ext* ext, int 
     I.N = N;
     I.stale = (ext->quirks & TTSH_QUIRK_STALE_HALO) ? 1 : 0;
     I.k2mode = ext->k2_mode;
-    int m = N, ns = 0;
-    while (m % 4 == 0) { I.radix[ns++] = 4; m /= 4; }
-    while (m % 2 == 0) { I.radix[ns++] = 2; m /= 2; }
-    while (m % 3 == 0) { I.radix[ns++] = 3; m /= 3; }
-    while (m % 5 == 0) { I.radix[ns++] = 5; m /= 5; }
-    I.nstages = ns;
+    int m = N;
+    std::vector<int> plan;
+    for (int r : {4, 2, 3, 5})
+      while (m % r == 0) { plan.push_back(r); m /= r; }
+    I.nstages = (int)plan.size();
+    for (size_t k = 0; k < plan.size(); ++k) I.radix[k] = plan[k];
+    fft_steps<double>(N, plan, I.step, &I.nsteps);
     Phys<double>& p = I.ph;
     p.h = h; p.dt = in->dt0; p.inv_dt = 1.0 / in->dt0;
     p.mu = in->mu; p.cA = in->cA; p.alpha = in->alpha; p.beta = in->beta; p.eta = in->eta;
@@ -211,11 +213,15 @@ extern "C" int ttsh_step_noalloc(const ttsh_input* in, const ttsh_ext* ext, int 
     k_noalloc_setup<<<1, 128, 0, st>>>(su, d_inst, d_tw, d_kval);
     NA_CK(cudaGetLastError());
     Group<double> g{d_inst, 1, N};
+    g.fft_kind = 2;
+    g.fft_nsteps = I.nsteps;
     for (int t = 0; t < nsteps; ++t) {
       launch_stage1<double>(g, 0, st);
       launch_stage2<double>(g, 0, st);
       launch_div<double>(g, 0, st);
-      for (int pass = 0; pass < 5; ++pass) launch_fft_pass<double>(g, pass, st);
+      launch_fft_plane<double>(g, 0, st);
+      launch_fft_pass<double>(g, 2, st);
+      launch_fft_plane<double>(g, 1, st);
       launch_correct<double>(g, 0, st);
       // the new phi, u*, P* become the caller's state (u*, P* feed the next step's stale halo)
       NA_CK(cudaMemcpyAsync(phi, phi_new, n * sizeof(double), cudaMemcpyDeviceToDevice, st));

@@ -121,6 +121,18 @@ __device__ __forceinline__ void record_wmax(int* wmax, float ax, float ay) {
   }
 }
 
+// The diagnostics' partials of a droplet: STATS_BLOCKS x {sum of phi, max |D.u|, max |u|, non-finite
+// values}. Adds a block's maxima (bits of non-negative doubles, which order as integers) and count
+// to one of them, chosen by `k`.
+constexpr int STATS_BLOCKS = 256;
+template <class T>
+__device__ __forceinline__ void stats_add(const InstDev<T>& I, int k, long long mdiv, long long mu, int bad) {
+  double* const out = I.red + 4 * (k % STATS_BLOCKS);
+  atomicMax(reinterpret_cast<long long*>(out + 1), mdiv);
+  atomicMax(reinterpret_cast<long long*>(out + 2), mu);
+  if (bad) atomicAdd(out + 3, (double)bad);
+}
+
 // Accessor of a scalar field around (x,y,z) with periodic wrap.
 template <class T>
 struct Acc {

@@ -51,6 +51,10 @@ template <> void launch_correct<double>(const Group<double>&, int, cudaStream_t)
 // FP64 diagnostics: per-instance partials into d_inst[i].red (nblocks_out per instance).
 template <class T> int launch_stats(const Group<T>& g, int par, cudaStream_t st, bool full = true);
 int stats_partials_per_instance(int N);
+// ... the part of the diagnostics that needs u and P, after the mass's
+template <class T> void launch_stats_u(const Group<T>& g, int par, cudaStream_t st);
+template <> void launch_stats_u<float>(const Group<float>&, int, cudaStream_t);
+template <> void launch_stats_u<double>(const Group<double>&, int, cudaStream_t);
 
 // Poisson solve by FFT (fft.cu): W <- (inverse FFT of -FFT(W)/k^2) / N^3.
 // pass 0: forward x; 1: forward y; 2: forward z, divide, inverse z; 3: inverse y; 4: inverse x + scale.

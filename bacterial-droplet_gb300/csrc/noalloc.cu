@@ -83,6 +83,27 @@ __global__ void k_noalloc_setup(const Setup s, ttsh::InstDev<double>* d_inst, do
   if (threadIdx.x == 0) *d_inst = s.inst;
 }
 
+// After a step: phi', u*', P*' into the caller's arrays, and (p_v non-null) the pressures, the real and
+// imaginary parts of W. One launch instead of three copies and two element-wise strided ones: a 32^3
+// call of one step 160 -> 112 us.
+__global__ void __launch_bounds__(256) k_noalloc_finish(const ttsh::InstDev<double>* __restrict__ inst, int n, double* __restrict__ p_v,
+                                                        double* __restrict__ p_p) {
+  const ttsh::InstDev<double>& I = *inst;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  I.phi[0][i] = I.phi[1][i];
+#pragma unroll
+  for (int b = 0; b < 3; ++b) {
+    I.Us[0][b][i] = I.Us[1][b][i];
+    I.Ps[0][b][i] = I.Ps[1][b][i];
+  }
+  if (p_v) {
+    const double2 w = I.W[i];
+    p_v[i] = w.x;
+    p_p[i] = w.y;
+  }
+}
+
 // Once per device (that device current): the device address of g_noalloc_scratch.
 int noalloc_scratch_address(int dev, unsigned char** out) {
   std::lock_guard<std::mutex> lk(g_mu);
@@ -223,17 +244,10 @@ extern "C" int ttsh_step_noalloc(const ttsh_input* in, const ttsh_ext* ext, int 
       launch_fft_pass<double>(g, 2, st);
       launch_fft_plane<double>(g, 1, st);
       launch_correct<double>(g, 0, st);
-      // the new phi, u*, P* become the caller's state (u*, P* feed the next step's stale halo)
-      NA_CK(cudaMemcpyAsync(phi, phi_new, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
-      NA_CK(cudaMemcpyAsync(ustar, us_new, 3 * n * sizeof(double), cudaMemcpyDeviceToDevice, st));
-      NA_CK(cudaMemcpyAsync(Pstar, ps_new, 3 * n * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    }
-    if (nsteps > 0) {
-      // pressures: real and imaginary parts of the packed field W
-      NA_CK(cudaMemcpy2DAsync(p_v, sizeof(double), I.W, 2 * sizeof(double), sizeof(double), n,
-                              cudaMemcpyDeviceToDevice, st));
-      NA_CK(cudaMemcpy2DAsync(p_p, sizeof(double), reinterpret_cast<double*>(I.W) + 1, 2 * sizeof(double),
-                              sizeof(double), n, cudaMemcpyDeviceToDevice, st));
+      // the new phi, u*, P* become the caller's state (u*, P* feed the next step's stale halo), and after
+      // the last step the pressures come out of the packed field
+      k_noalloc_finish<<<(int)((n + 255) / 256), 256, 0, st>>>(d_inst, (int)n, t + 1 == nsteps ? p_v : nullptr, p_p);
+      NA_CK(cudaGetLastError());
     }
     NA_CK(cudaGetLastError());
 #undef NA_CK

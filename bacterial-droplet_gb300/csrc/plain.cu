@@ -11,6 +11,8 @@
 #include <algorithm>
 #include <cstdio>
 #include <stdexcept>
+#include <string>
+#include <utility>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -30,157 +32,279 @@ inline void check_launch(const char* what) {
   }
 }
 
-inline dim3 site_grid(int N, int n) {
-  if ((long)N * n > 65535) throw std::runtime_error("too many instances of this size in one group");
-  return dim3((N + BX - 1) / BX, (N + BY - 1) / BY, N * n);
-}
+// ---- staged planes ---------------------------------------------------------------------------
+// The kernels evaluate the reference's stencils in its arithmetic order, one thread per site of a
+// 32 x 8 column tile, and march along z: the planes z-1, z, z+1 of every field a kernel's stencils
+// read (tile + 1) lie in a ring of planes in shared memory, into which the next ones are copied
+// (cp.async) meanwhile. With each neighbour read from global memory instead, a site of k_stage2
+// loaded some 600 values through L1, each with its own 64-bit address: 4 x 100^3, us per launch,
+// k_stage1 144 -> 126, k_stage2 1178 -> 519, k_div 311 -> 114, k_correct 125 -> 81. They are now bound by
+// shared-memory reads (79 - 91 % of the pipe). All of a site's arithmetic follows one barrier, so that
+// it stays one expression with the roundings it has always had.
+constexpr int SX = BX + 2, SYR = BY + 2, SPL = SX * SYR, NT = BX * BY;
 
-template <class T>
-__global__ void __launch_bounds__(BX* BY) k_stage1(const InstDev<T>* __restrict__ insts, int par) {
-  const int N = insts[0].N;
-  const InstDev<T>& I = insts[blockIdx.z / N];
-  const int z = blockIdx.z % N;
-  const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y;
-  // FP32: this step's maxima of the Poisson source start from zero (k_div records them)
-  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.y == 0 && I.wmax)
-    for (int i = threadIdx.x; i < 2 * (int)(gridDim.z / N); i += blockDim.x) insts[i >> 1].wmax[i & 1] = 0;
-  if (x >= N || y >= N) return;
-  Site s;
-  s.init(x, y, z, N);
-  const Phys<T>& p = I.ph;
-  const T* phi = I.phi[par];
-  const T ph = phi[s.idx];
-  // mu_0 (TTSH3D.cu:567)
-  I.mu0[s.idx] = p.aPhi2 * (ph - 3 * ph * ph + 2 * ph * ph * ph) - p.kPhi * st_lap<T>(s.acc(phi), p);
-#pragma unroll
-  for (int b = 0; b < 3; ++b) {
-    Acc<T> F = s.acc<T>(I.P[b]);
-    // mu_b (:571-573)
-    I.mu[b][s.idx] = ph * I.P[b][s.idx] + p.La2 * st_lap<T>(F, p);
-    // sigma_ab = phi * D_a P_b (:587-595; the 1/28 term is an integer-division zero)
-    I.sig[0 * 3 + b][s.idx] = ph * st_dx<T>(F, p.c2h);
-    I.sig[1 * 3 + b][s.idx] = ph * st_dy<T>(F, p.c2h);
-    I.sig[2 * 3 + b][s.idx] = ph * st_dz<T>(F, p.c2h);
-  }
-}
+// NF fields of elements E (float; float2: an interleaved complex field), RING slots.
+template <class E, int NF, int RING>
+struct Planes {
+  E* sm;               // [RING][NF][SPL]
+  int N, NN, z0, tid;
+  int go[2];           // this thread's staged points (two at most): offset within a plane, or -1
+  bool out[2];         // ... beyond the boundary in x or y
+  int lx, ly, x, y;
 
-template <class T>
-__global__ void __launch_bounds__(BX* BY) k_stage2(const InstDev<T>* __restrict__ insts, int par) {
-  const int N = insts[0].N;
-  const InstDev<T>& I = insts[blockIdx.z / N];
-  const int z = blockIdx.z % N;
-  const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y;
-  if (x >= N || y >= N) return;
-  Site s;
-  s.init(x, y, z, N);
-  const Phys<T>& p = I.ph;
-  const int i = s.idx;
-  const T* phi = I.phi[par];
-  Acc<T> Fphi = s.acc(phi);
-  const T dphi[3] = {st_dx<T>(Fphi, p.c2h), st_dy<T>(Fphi, p.c2h), st_dz<T>(Fphi, p.c2h)};
-  const T vx = I.U[0][i], vy = I.U[1][i], vz = I.U[2][i];
-  const T px = I.P[0][i], py = I.P[1][i], pz = I.P[2][i], ph = phi[i];
-  const T P2 = px * px + py * py + pz * pz;
-  const T dPhi2 = dphi[0] * dphi[0] + dphi[1] * dphi[1] + dphi[2] * dphi[2];
-  const T mu0 = I.mu0[i];
-  // getDtF, velocity (TTSH3D.cu:617-621) and getVStar (:480-482)
+  static constexpr size_t bytes() { return (size_t)RING * NF * SPL * sizeof(E); }
+  __device__ __forceinline__ Planes(unsigned char* m, int N_, int z0_) : sm(reinterpret_cast<E*>(m)), N(N_), NN(N_ * N_), z0(z0_) {
+    tid = threadIdx.x;
+    lx = tid & 31;
+    ly = tid >> 5;
+    const int x0 = blockIdx.x * BX, y0 = blockIdx.y * BY;
+    x = x0 + lx;
+    y = y0 + ly;
 #pragma unroll
-  for (int b = 0; b < 3; ++b) {
-    Acc<T> Fv = s.acc<T>(I.U[b]);
-    T r = -vx * st_dx<T>(Fv, p.c2h) - vy * st_dy<T>(Fv, p.c2h) - vz * st_dz<T>(Fv, p.c2h) + p.mu * st_lap<T>(Fv, p) +
-          mu0 * dphi[b] +
-          p.cA * (st_dx<T>(s.acc<T>(I.sig[0 * 3 + b]), p.c2h) + st_dy<T>(s.acc<T>(I.sig[1 * 3 + b]), p.c2h) +
-                  st_dz<T>(s.acc<T>(I.sig[2 * 3 + b]), p.c2h));
-    if (p.zeta != T(0)) {
-      r = r - p.zeta * (st_dx<T>(s.acc_prod<T>(phi, I.P[0], I.P[b]), p.c2h) +
-                        st_dy<T>(s.acc_prod<T>(phi, I.P[1], I.P[b]), p.c2h) +
-                        st_dz<T>(s.acc_prod<T>(phi, I.P[2], I.P[b]), p.c2h));
+    for (int k = 0; k < 2; ++k) {
+      const int i = tid + k * NT, r = i / SX, gx = x0 - 1 + i - r * SX, gy = y0 - 1 + r;
+      // a partial tile's points beyond its halo wrap too (small boxes more than once); they are not used
+      go[k] = i < SPL ? wrapi(gy, N) % N * N + wrapi(gx, N) % N : -1;
+      out[k] = gx < 0 || gx >= N || gy < 0 || gy >= N;
     }
-    const T u = b == 0 ? vx : (b == 1 ? vy : vz);
-    I.Us[par ^ 1][b][i] = u + p.dt * r;
   }
-  // getDtF, polarisation (:623-629) and getVStar (:486-488)
-  const T pb[3] = {px, py, pz};
+  __device__ __forceinline__ bool on() const { return x < N && y < N; }
+  __device__ __forceinline__ int slot(int z) const { return (z - z0 + 1) % RING; }
+  // copies plane z; src(f, beyond) is the array field f's values come from, `beyond` where the point lies
+  // beyond the boundary
+  template <class F>
+  __device__ __forceinline__ void stage(int z, F&& src, bool any) const {
+    const size_t zo = (size_t)wrapi(z, N) * NN;
+    const bool zw = z < 0 || z >= N;
 #pragma unroll
-  for (int b = 0; b < 3; ++b) {
-    Acc<T> Fp = s.acc<T>(I.P[b]);
-    const T dxp = st_dx<T>(Fp, p.c2h), dyp = st_dy<T>(Fp, p.c2h), dzp = st_dz<T>(Fp, p.c2h);
-    T cub;
-    if (b == 0) cub = px * px * px + px * py * py + px * pz * pz;
-    else if (b == 1) cub = px * py * px + py * py * py + py * pz * pz;
-    else cub = px * pz * px + py * pz * py + pz * pz * pz;
-    const T Ab = dphi[0] * dphi[b] * px + dphi[1] * dphi[b] * py + dphi[2] * dphi[b] * pz;
-    // OP_b + kappa*phi*DP_b are integer-division zeros in the reference (:579-585).
-    const T r = -vx * dxp - vy * dyp - vz * dzp - p.alpha * ph * pb[b] - p.beta * P2 * pb[b] +
-                p.eta * st_lap<T>(s.acc<T>(I.mu[b]), p) - p.lambda0 * (px * dxp + py * dyp + pz * dzp) -
-                p.A * (dPhi2 * cub + sqrt(P2) * Ab);
-    I.Ps[par ^ 1][b][i] = pb[b] + p.dt * r;
-  }
-  // dtphi (:631) and the phi update of getVNew (:515)
-  const T dtphi = -vx * dphi[0] - vy * dphi[1] - vz * dphi[2] + p.gamma * (st_lap<T>(s.acc<T>(I.mu0), p));
-  I.phi[par ^ 1][i] = ph + p.dt * dtphi;
-}
-
-template <class T>
-__global__ void __launch_bounds__(BX* BY) k_div(const InstDev<T>* __restrict__ insts, int par) {
-  const int N = insts[0].N;
-  const InstDev<T>& I = insts[blockIdx.z / N];
-  const int z = blockIdx.z % N;
-  const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y;
-  if (x >= N || y >= N) return;
-  Site s;
-  s.init(x, y, z, N);
-  const Phys<T>& p = I.ph;
-  T d[2];
+    for (int k = 0; k < 2; ++k) {
+      if (go[k] < 0 || !any) continue;
+      E* d = sm + (size_t)slot(z) * NF * SPL + tid + k * NT;
 #pragma unroll
-  for (int f = 0; f < 2; ++f) {
-    T* const* cur = f == 0 ? I.Us[par ^ 1] : I.Ps[par ^ 1];
-    T* const* old = f == 0 ? I.Us[par] : I.Ps[par];
-    T a, b, c;
-    if (I.stale) {
-      a = st_dx<T>(s.acc_stale<T>(cur[0], old[0]), p.c2h);
-      b = st_dy<T>(s.acc_stale<T>(cur[1], old[1]), p.c2h);
-      c = st_dz<T>(s.acc_stale<T>(cur[2], old[2]), p.c2h);
-    } else {
-      a = st_dx<T>(s.acc<T>(cur[0]), p.c2h);
-      b = st_dy<T>(s.acc<T>(cur[1]), p.c2h);
-      c = st_dz<T>(s.acc<T>(cur[2]), p.c2h);
+      for (int f = 0; f < NF; ++f) {
+        const E* g = src(f, zw || out[k]) + zo + go[k];
+        const unsigned a = (unsigned)__cvta_generic_to_shared(d + f * SPL);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(a), "l"(g), "n"(sizeof(E)) : "memory");
+      }
     }
-    d[f] = (a + b + c) * p.inv_dt;  // getStream mode 0 (:666-668)
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
   }
-  typename CxT<T>::type w;
-  w.x = d[0];
-  w.y = d[1];
-  I.W[s.idx] = w;
-  if constexpr (sizeof(T) == 4) record_wmax(I.wmax, d[0], d[1]);
+  // body(z) for the planes z0 .. z1 - 1, each after its neighbours have arrived
+  template <class F, class G>
+  __device__ __forceinline__ void march(int z1, F&& src, G&& body) const {
+#pragma unroll 1
+    for (int z = z0 - 1; z < z0 + RING - 2; ++z) stage(z <= z1 ? z : z1, src, z <= z1);
+    for (int z = z0; z < z1; ++z) {
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(RING - 4) : "memory");  // planes up to z + 1
+      __syncthreads();  // the planes of every thread; and plane z - 2 has been read
+      stage(z + RING - 2, src, z + RING - 2 <= z1);
+      if (on()) body(z);
+    }
+  }
+  // this thread's site in field 0 of plane z
+  __device__ __forceinline__ const E* at(int z) const { return sm + (size_t)slot(z) * NF * SPL + (ly + 1) * SX + lx + 1; }
+};
+
+// Accessors of staged fields for st_dx .. st_lap: p[1 + dz] is the site in the planes z-1, z, z+1; or
+// the 27 values in registers.
+struct AccS {
+  const float* p[3];
+  __device__ __forceinline__ float operator()(int dx, int dy, int dz) const { return p[dz + 1][dy * SX + dx]; }
+};
+struct AccV {
+  float v[27];
+  __device__ __forceinline__ float operator()(int dx, int dy, int dz) const { return v[(dz + 1) * 9 + (dy + 1) * 3 + dx + 1]; }
+};
+// the pointwise product phi * Pa * Pb (build-defined active stress)
+struct AccProd {
+  AccS phi, pa, pb;
+  __device__ __forceinline__ float operator()(int dx, int dy, int dz) const { return phi(dx, dy, dz) * pa(dx, dy, dz) * pb(dx, dy, dz); }
+};
+template <int NF, int RING>
+__device__ __forceinline__ AccS field(const Planes<float, NF, RING>& P, int z, int f) {
+  return AccS{{P.at(z - 1) + f * SPL, P.at(z) + f * SPL, P.at(z + 1) + f * SPL}};
 }
 
-template <class T>
-__global__ void __launch_bounds__(BX* BY) k_correct(const InstDev<T>* __restrict__ insts, int par) {
+typedef InstDev<float> Inst;
+typedef float T;
+
+__global__ void __launch_bounds__(NT, 4) k_stage1(const Inst* __restrict__ insts, int par, int nchunk, int zc) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const int N = insts[0].N;
-  const InstDev<T>& I = insts[blockIdx.z / N];
-  const int z = blockIdx.z % N;
-  const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y;
-  if (x >= N || y >= N) return;
-  Site s;
-  s.init(x, y, z, N);
+  const Inst& I = insts[blockIdx.z / nchunk];
+  // this step's maxima of the Poisson source start from zero (k_div records them)
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)
+    for (int i = threadIdx.x; i < 2 * (int)(gridDim.z / nchunk); i += blockDim.x) insts[i >> 1].wmax[i & 1] = 0;
+  const int z0 = (blockIdx.z % nchunk) * zc;
+  const Planes<float, 4, 7> S(smem_raw, N, z0);
   const Phys<T>& p = I.ph;
-  const T* W = reinterpret_cast<const T*>(I.W);
-  Acc<T> Fv = s.acc<T>(W, 2), Fp = s.acc<T>(W + 1, 2);
-  const int i = s.idx;
-  // FP32: the pressures come out of the FFT scaled by powers of two (pow2_norm); undo it exactly
-  T du = T(1), dp = T(1);
-  if constexpr (sizeof(T) == 4) {
-    du = pow2_denorm(I.wmax[0]);
-    dp = pow2_denorm(I.wmax[1]);
-  }
-  // getVNew (TTSH3D.cu:505-511)
-  I.U[0][i] = I.Us[par ^ 1][0][i] - p.dt * (st_dx<T>(Fv, p.c2h) * du);
-  I.U[1][i] = I.Us[par ^ 1][1][i] - p.dt * (st_dy<T>(Fv, p.c2h) * du);
-  I.U[2][i] = I.Us[par ^ 1][2][i] - p.dt * (st_dz<T>(Fv, p.c2h) * du);
-  I.P[0][i] = I.Ps[par ^ 1][0][i] - p.dt * (st_dx<T>(Fp, p.c2h) * dp);
-  I.P[1][i] = I.Ps[par ^ 1][1][i] - p.dt * (st_dy<T>(Fp, p.c2h) * dp);
-  I.P[2][i] = I.Ps[par ^ 1][2][i] - p.dt * (st_dz<T>(Fp, p.c2h) * dp);
+  auto src = [&](int f, bool) -> const float* { return f == 0 ? I.phi[par] : I.P[f - 1]; };
+  S.march(min(z0 + zc, N), src, [&](int z) {
+    const int i = z * S.NN + S.y * N + S.x;
+    const AccS phi = field(S, z, 0);
+    const T ph = phi(0, 0, 0);
+    // mu_0 (TTSH3D.cu:567)
+    const T mu0 = p.aPhi2 * (ph - 3 * ph * ph + 2 * ph * ph * ph) - p.kPhi * st_lap<T>(phi, p);
+    T mu[3], sig[9];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      const AccS F = field(S, z, b + 1);
+      // mu_b (:571-573)
+      mu[b] = ph * F(0, 0, 0) + p.La2 * st_lap<T>(F, p);
+      // sigma_ab = phi * D_a P_b (:587-595; the 1/28 term is an integer-division zero)
+      sig[0 * 3 + b] = ph * st_dx<T>(F, p.c2h);
+      sig[1 * 3 + b] = ph * st_dy<T>(F, p.c2h);
+      sig[2 * 3 + b] = ph * st_dz<T>(F, p.c2h);
+    }
+    // the stores after the last stencil: a store may alias the staged values, which are then read again
+    I.mu0[i] = mu0;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) I.mu[b][i] = mu[b];
+#pragma unroll
+    for (int b = 0; b < 9; ++b) I.sig[b][i] = sig[b];
+  });
+}
+
+// fields: phi, P (1 + b), u (4 + b), mu_0 (7), mu_b (8 + b), sigma_ab (11 + 3 a + b)
+__global__ void __launch_bounds__(NT, 2) k_stage2(const Inst* __restrict__ insts, int par, int nchunk, int zc) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int N = insts[0].N;
+  const Inst& I = insts[blockIdx.z / nchunk];
+  const int z0 = (blockIdx.z % nchunk) * zc;
+  const Planes<float, 20, 4> S(smem_raw, N, z0);
+  const Phys<T>& p = I.ph;
+  auto src = [&](int f, bool) -> const float* {
+    return f == 0 ? I.phi[par] : (f < 4 ? I.P[f - 1] : (f < 7 ? I.U[f - 4] : (f == 7 ? I.mu0 : (f < 11 ? I.mu[f - 8] : I.sig[f - 11]))));
+  };
+  S.march(min(z0 + zc, N), src, [&](int z) {
+    const int i = z * S.NN + S.y * N + S.x;
+    auto F = [&](int f) { return field(S, z, f); };
+    const AccS Fphi = F(0);
+    const T dphi[3] = {st_dx<T>(Fphi, p.c2h), st_dy<T>(Fphi, p.c2h), st_dz<T>(Fphi, p.c2h)};
+    const T vx = F(4)(0, 0, 0), vy = F(5)(0, 0, 0), vz = F(6)(0, 0, 0);
+    const T px = F(1)(0, 0, 0), py = F(2)(0, 0, 0), pz = F(3)(0, 0, 0), ph = Fphi(0, 0, 0);
+    const T P2 = px * px + py * py + pz * pz;
+    const T dPhi2 = dphi[0] * dphi[0] + dphi[1] * dphi[1] + dphi[2] * dphi[2];
+    const T mu0 = F(7)(0, 0, 0);
+    T us[3], ps[3];
+    // getDtF, velocity (TTSH3D.cu:617-621) and getVStar (:480-482)
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      const AccS Fv = F(4 + b);
+      T r = -vx * st_dx<T>(Fv, p.c2h) - vy * st_dy<T>(Fv, p.c2h) - vz * st_dz<T>(Fv, p.c2h) + p.mu * st_lap<T>(Fv, p) +
+            mu0 * dphi[b] +
+            p.cA * (st_dx<T>(F(11 + b), p.c2h) + st_dy<T>(F(14 + b), p.c2h) + st_dz<T>(F(17 + b), p.c2h));
+      if (p.zeta != T(0)) {
+        r = r - p.zeta * (st_dx<T>(AccProd{Fphi, F(1), F(1 + b)}, p.c2h) + st_dy<T>(AccProd{Fphi, F(2), F(1 + b)}, p.c2h) +
+                          st_dz<T>(AccProd{Fphi, F(3), F(1 + b)}, p.c2h));
+      }
+      const T u = b == 0 ? vx : (b == 1 ? vy : vz);
+      us[b] = u + p.dt * r;
+    }
+    // getDtF, polarisation (:623-629) and getVStar (:486-488)
+    const T pb[3] = {px, py, pz};
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      const AccS Fp = F(1 + b);
+      const T dxp = st_dx<T>(Fp, p.c2h), dyp = st_dy<T>(Fp, p.c2h), dzp = st_dz<T>(Fp, p.c2h);
+      T cub;
+      if (b == 0) cub = px * px * px + px * py * py + px * pz * pz;
+      else if (b == 1) cub = px * py * px + py * py * py + py * pz * pz;
+      else cub = px * pz * px + py * pz * py + pz * pz * pz;
+      const T Ab = dphi[0] * dphi[b] * px + dphi[1] * dphi[b] * py + dphi[2] * dphi[b] * pz;
+      // OP_b + kappa*phi*DP_b are integer-division zeros in the reference (:579-585).
+      const T r = -vx * dxp - vy * dyp - vz * dzp - p.alpha * ph * pb[b] - p.beta * P2 * pb[b] +
+                  p.eta * st_lap<T>(F(8 + b), p) - p.lambda0 * (px * dxp + py * dyp + pz * dzp) -
+                  p.A * (dPhi2 * cub + sqrt(P2) * Ab);
+      ps[b] = pb[b] + p.dt * r;
+    }
+    // dtphi (:631) and the phi update of getVNew (:515)
+    const T dtphi = -vx * dphi[0] - vy * dphi[1] - vz * dphi[2] + p.gamma * (st_lap<T>(F(7), p));
+    I.phi[par ^ 1][i] = ph + p.dt * dtphi;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      I.Us[par ^ 1][b][i] = us[b];
+      I.Ps[par ^ 1][b][i] = ps[b];
+    }
+  });
+}
+
+// fields: u*_a (a), P*_a (3 + a); beyond the boundary the previous step's (quirk Q2 of the reference:
+// the halo of u*, P* is refreshed at the start of getRHS, TTSH3D.cu:369-371 and :405-407, before
+// getVStar rewrites the interior, :471-491)
+__global__ void __launch_bounds__(NT, 4) k_div(const Inst* __restrict__ insts, int par, int nchunk, int zc) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int N = insts[0].N;
+  const Inst& I = insts[blockIdx.z / nchunk];
+  const int z0 = (blockIdx.z % nchunk) * zc;
+  const Planes<float, 6, 6> S(smem_raw, N, z0);
+  const Phys<T>& p = I.ph;
+  const bool stale = I.stale;
+  auto src = [&](int f, bool beyond) -> const float* {
+    const int q = stale && beyond ? par : par ^ 1;
+    return f < 3 ? I.Us[q][f] : I.Ps[q][f - 3];
+  };
+  T mx = 0, my = 0;
+  S.march(min(z0 + zc, N), src, [&](int z) {
+    T d[2];
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+      const T a = st_dx<T>(field(S, z, 3 * f), p.c2h);
+      const T b = st_dy<T>(field(S, z, 3 * f + 1), p.c2h);
+      const T c = st_dz<T>(field(S, z, 3 * f + 2), p.c2h);
+      d[f] = (a + b + c) * p.inv_dt;  // getStream mode 0 (:666-668)
+    }
+    I.W[z * S.NN + S.y * N + S.x] = make_float2(d[0], d[1]);
+    mx = fmaxf(mx, fabsf(d[0]));
+    my = fmaxf(my, fabsf(d[1]));
+  });
+  record_wmax(I.wmax, mx, my);
+}
+
+__global__ void __launch_bounds__(NT, 5) k_correct(const Inst* __restrict__ insts, int par, int nchunk, int zc) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int N = insts[0].N;
+  const Inst& I = insts[blockIdx.z / nchunk];
+  const int z0 = (blockIdx.z % nchunk) * zc;
+  const Planes<float2, 1, 8> S(smem_raw, N, z0);
+  const Phys<T>& p = I.ph;
+  // the pressures come out of the FFT scaled by powers of two (pow2_norm); undo it exactly
+  const T du = pow2_denorm(I.wmax[0]), dp = pow2_denorm(I.wmax[1]);
+  auto src = [&](int, bool) -> const float2* { return I.W; };
+  S.march(min(z0 + zc, N), src, [&](int z) {
+    const int i = z * S.NN + S.y * N + S.x;
+    // both pressures of a neighbour by one 8-byte load
+    AccV Fv, Fp;
+#pragma unroll
+    for (int k = 0; k < 27; ++k) {
+      const float2 w = S.at(z - 1 + k / 9)[(k / 3 % 3 - 1) * SX + k % 3 - 1];
+      Fv.v[k] = w.x;
+      Fp.v[k] = w.y;
+    }
+    // getVNew (TTSH3D.cu:505-511)
+    const T u[3] = {I.Us[par ^ 1][0][i] - p.dt * (st_dx<T>(Fv, p.c2h) * du), I.Us[par ^ 1][1][i] - p.dt * (st_dy<T>(Fv, p.c2h) * du),
+                    I.Us[par ^ 1][2][i] - p.dt * (st_dz<T>(Fv, p.c2h) * du)};
+    const T P[3] = {I.Ps[par ^ 1][0][i] - p.dt * (st_dx<T>(Fp, p.c2h) * dp), I.Ps[par ^ 1][1][i] - p.dt * (st_dy<T>(Fp, p.c2h) * dp),
+                    I.Ps[par ^ 1][2][i] - p.dt * (st_dz<T>(Fp, p.c2h) * dp)};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      I.U[k][i] = u[k];
+      I.P[k][i] = P[k];
+    }
+  });
+}
+
+// Planes per CTA: 16 (three planes beyond them are staged), halved while the grid has fewer than
+// four CTAs per SM.
+template <class K>
+void launch_planes(K kernel, size_t smem, const Group<float>& g, int par, cudaStream_t st, const char* what) {
+  if ((long)g.N * g.n > 65535) throw std::runtime_error("too many instances of this size in one group");
+  const int nx = (g.N + BX - 1) / BX, ny = (g.N + BY - 1) / BY;
+  int zc = std::min(16, g.N);
+  while (zc > 1 && (long)nx * ny * g.n * ((g.N + zc - 1) / zc) < 608) zc /= 2;
+  const int nchunk = (g.N + zc - 1) / zc;
+  kernel<<<dim3(nx, ny, nchunk * g.n), NT, smem, st>>>(g.d_inst, par, nchunk, zc);
+  check_launch(what);
 }
 
 constexpr int STATS_THREADS = 256;
@@ -192,7 +316,7 @@ constexpr int STATS_THREADS = 256;
 // only the per-thread partials are combined in FP64: the GPU's FP64 rate is a small fraction of
 // its FP32 rate, and an FP64 add per site would cost more than the step's stencils for a mass
 // read-back after every step. The maxima are exact in either precision.
-template <class T>
+template <class V>
 struct MassAcc;
 template <>
 struct MassAcc<double> {
@@ -293,11 +417,6 @@ __global__ void __launch_bounds__(STATS_THREADS) k_stats_mass(const InstDev<T>* 
 // zc planes; the three components' planes (tile + 1) go through a ring of three in shared memory, so
 // that each value is read once from global memory per tile instead of up to 27 times, with no
 // integer divisions per site: 160^3 with the mass 272 -> 76 us, 2 x 256^3 1106 -> 416 us.
-constexpr int SX = BX + 2, SYR = BY + 2, SPL = SX * SYR;
-struct AccS {  // st_dx .. of common.cuh over the staged planes z - 1, z, z + 1
-  const float* p[3];
-  __device__ __forceinline__ float operator()(int dx, int dy, int dz) const { return p[dz + 1][dy * SX + dx]; }
-};
 __global__ void __launch_bounds__(BX* BY) k_stats_u(const InstDev<float>* __restrict__ insts, int nchunk, int zc) {
   __shared__ float ring[3][3][SPL];
   const InstDev<float>& I = insts[blockIdx.z / nchunk];
@@ -375,25 +494,32 @@ __global__ void __launch_bounds__(BX* BY) k_stats_u(const InstDev<float>* __rest
 
 int stats_partials_per_instance(int) { return STATS_BLOCKS; }
 
+void plain32_prepare() {
+  const std::pair<const void*, size_t> k[] = {{(const void*)k_stage1, Planes<float, 4, 7>::bytes()},
+                                              {(const void*)k_stage2, Planes<float, 20, 4>::bytes()},
+                                              {(const void*)k_div, Planes<float, 6, 6>::bytes()},
+                                              {(const void*)k_correct, Planes<float2, 1, 8>::bytes()}};
+  for (const auto& f : k) {
+    const cudaError_t e = cudaFuncSetAttribute(f.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.second);
+    if (e != cudaSuccess) throw std::runtime_error(std::string("plain kernels' smem attribute: ") + cudaGetErrorString(e));
+  }
+}
+
 template <>
 void launch_stage1<float>(const Group<float>& g, int par, cudaStream_t st) {
-  k_stage1<float><<<site_grid(g.N, g.n), dim3(BX, BY), 0, st>>>(g.d_inst, par);
-  check_launch("stage1");
+  launch_planes(k_stage1, Planes<float, 4, 7>::bytes(), g, par, st, "stage1");
 }
 template <>
 void launch_stage2<float>(const Group<float>& g, int par, cudaStream_t st) {
-  k_stage2<float><<<site_grid(g.N, g.n), dim3(BX, BY), 0, st>>>(g.d_inst, par);
-  check_launch("stage2");
+  launch_planes(k_stage2, Planes<float, 20, 4>::bytes(), g, par, st, "stage2");
 }
 template <>
 void launch_div<float>(const Group<float>& g, int par, cudaStream_t st) {
-  k_div<float><<<site_grid(g.N, g.n), dim3(BX, BY), 0, st>>>(g.d_inst, par);
-  check_launch("div");
+  launch_planes(k_div, Planes<float, 6, 6>::bytes(), g, par, st, "div");
 }
 template <>
 void launch_correct<float>(const Group<float>& g, int par, cudaStream_t st) {
-  k_correct<float><<<site_grid(g.N, g.n), dim3(BX, BY), 0, st>>>(g.d_inst, par);
-  check_launch("correct");
+  launch_planes(k_correct, Planes<float2, 1, 8>::bytes(), g, par, st, "correct");
 }
 template <>
 void launch_stats_u<float>(const Group<float>& g, int, cudaStream_t st) {

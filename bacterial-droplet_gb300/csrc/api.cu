@@ -620,6 +620,7 @@ void set_radix(ttsh_sim* s, Engine<T>& E, size_t gi, const std::vector<int>& r) 
     for (size_t k = 0; k < r.size(); ++k) E.h[i].radix[k] = r[k];
     fft_steps<T>(E.h[i].N, r, E.h[i].step, &E.h[i].nsteps);
     E.groups[gi].fft_nsteps = E.h[i].nsteps;
+    E.groups[gi].fft_default = r == radix_plan(E.h[i].N);
   }
   upload_group(s, E, gi);
 }

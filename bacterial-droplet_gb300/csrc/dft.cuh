@@ -22,7 +22,7 @@ __device__ __forceinline__ float2 axpy(float2 a, float s, float2 b) { return __f
 __device__ __forceinline__ float2 sub(float2 a, float2 b) { return axpy(a, -1.f, b); }
 template <class C>
 __device__ __forceinline__ C mul(C a, C b) {
-  return mk<C>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+  return mk<C>(fma(a.x, b.x, -(a.y * b.y)), fma(a.x, b.y, a.y * b.x));
 }
 template <class C>
 __device__ __forceinline__ C conj(C a) { return mk<C>(a.x, -a.y); }

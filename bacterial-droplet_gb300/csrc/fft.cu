@@ -31,28 +31,19 @@
 
 #include "common.cuh"
 #include "dft.cuh"
+#include "fftplan.h"
 #include "fftreg.cuh"
+#include "fftstage.cuh"
 #include "kernels.h"
 
 namespace ttsh {
 
 using fftreg::scale_n3;
+using namespace fftplan;
 
 namespace {
 
-constexpr int FFT_THREADS = 256;
-
-// a b in FP32: one product of each part is rounded, the other joins it in a fused multiply-add. INV (the
-// inverse transform, run on conjugated values) fuses the other product of the imaginary part: the
-// choice the compiler makes for a times a conjugated twiddle, which the results have always had.
-template <bool INV>
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(fmaf(a.x, b.x, -(a.y * b.y)), INV ? fmaf(a.y, b.x, a.x * b.y) : fmaf(a.x, b.y, a.y * b.x));
-}
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-
-template <class T> constexpr int fft_min_ctas() { return sizeof(T) == 4 ? 3 : 2; }
+constexpr int FFT_THREADS = fftplan::kThreads;
 
 // The smem position of element e of line l. Lines along x (contiguous in memory) are one after
 // another, elements spread by one in eight so that a step's stride-R writes use more banks; lines
@@ -61,7 +52,6 @@ template <bool XAXIS>
 __device__ __forceinline__ int spos(int l, int e, int LB, int pitch) {
   return XAXIS ? l * pitch + e + (e >> 3) : e * LB + l;
 }
-inline int x_pitch(int N) { return N + N / 8 + 1; }
 
 // One line group of a pass: where its lines are.
 struct Lines {
@@ -146,39 +136,6 @@ __device__ __forceinline__ void fft_step(const InstDev<double>& I, int pass, con
   }
 }
 
-// FP32: one butterfly of the radix plan, in place: the twiddles w^(r k ts) of its stage, then the DFT
-// of R = 2, 4 in butterflies, of R = 3, 5 as the sum that defines it (its roots of unity from the
-// table).
-template <bool INV, int R>
-__device__ __forceinline__ void plan_butterfly(float2* v, const float2* tw, int N, int k, int ts) {
-  if (k > 0) {
-#pragma unroll
-    for (int r = 1; r < R; ++r) v[r] = cmul<INV>(v[r], __ldg(tw + r * k * ts));
-  }
-  if constexpr (R == 2) {
-    const float2 a = v[0], b = v[1];
-    v[0] = cadd(a, b);
-    v[1] = csub(a, b);
-  } else if constexpr (R == 4) {
-    const float2 a = cadd(v[0], v[2]), b = csub(v[0], v[2]), c = cadd(v[1], v[3]), d = csub(v[1], v[3]);
-    const float2 dd = make_float2(d.y, -d.x);
-    v[0] = cadd(a, c);
-    v[2] = csub(a, c);
-    v[1] = cadd(b, dd);
-    v[3] = csub(b, dd);
-  } else {
-    float2 o[R];
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      float2 acc = v[0];
-#pragma unroll
-      for (int r = 1; r < R; ++r) acc = cadd(acc, cmul<INV>(v[r], __ldg(tw + ((q * r) % R) * (N / R))));
-      o[q] = acc;
-    }
-#pragma unroll
-    for (int q = 0; q < R; ++q) v[q] = o[q];
-  }
-}
 // FP32: the plan's stages R1 and (R2 > 1) R2 in one step. With P = N / (R1 R2), the thread of base j
 // holds the elements j + (r R2 + q) P: for each q the inputs (over r) of stage R1's butterfly j + q P,
 // whose outputs r are, for each r, the inputs (over q) of the stage-R2 butterfly (j / Ns) Ns R1 + k + r Ns.
@@ -202,20 +159,25 @@ __device__ __forceinline__ void fft_step(const InstDev<float>& I, int pass, cons
 #pragma unroll
       for (int r = 0; r < R1; ++r) v[r * R2 + q] = u[r];
     }
-    const fftreg::Poisson<float> pm(I, XAXIS ? 0 : L.x0 + l, XAXIS ? 0 : L.y);
+    if constexpr (R2 > 1) {
 #pragma unroll
-    for (int r = 0; r < R1; ++r) {
-      float2 u[R2];
+      for (int r = 0; r < R1; ++r) {
+        float2 u[R2];
 #pragma unroll
-      for (int q = 0; q < R2; ++q) u[q] = v[r * R2 + q];
-      if constexpr (R2 > 1) plan_butterfly<INV, R2>(u, I.tw, N, k + r * Ns, N / (Ns * R));
+        for (int q = 0; q < R2; ++q) u[q] = v[r * R2 + q];
+        plan_butterfly<INV, R2>(u, I.tw, N, k + r * Ns, N / (Ns * R));
 #pragma unroll
-      for (int q = 0; q < R2; ++q) {
-        const int e = e0 + r * Ns + q * Ns * R1;
-        if (!XAXIS && divide) u[q] = dft::conj(pm(u[q], I, e));
-        store<float, XAXIS>(u[q], I, pass, L, io, l, e);
+        for (int q = 0; q < R2; ++q) v[r * R2 + q] = u[q];
       }
     }
+    // v[r R2 + q] is element e0 + (r + q R1) Ns
+    if (!XAXIS && !INV && divide) {
+      const fftreg::Poisson<float> pm(I, L.x0 + l, L.y);
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = dft::conj(pm(v[r], I, e0 + (r / R2 + r % R2 * R1) * Ns));
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) store<float, XAXIS>(v[r], I, pass, L, io, l, e0 + (r / R2 + r % R2 * R1) * Ns);
   }
 }
 
@@ -231,8 +193,6 @@ __device__ __forceinline__ void run_step(int s, const InstDev<double>& I, int pa
     default: break;
   }
 }
-#define TTSH_STAGE_PAIRS(X) \
-  X(2, 1) X(3, 1) X(4, 1) X(5, 1) X(4, 4) X(4, 2) X(4, 3) X(4, 5) X(2, 3) X(2, 5) X(3, 3) X(3, 5) X(5, 5)
 template <bool XAXIS>
 __device__ __forceinline__ void run_step(int s, const InstDev<float>& I, int pass, const Lines& L, const Io<float2>& io, int Ns, bool divide,
                                          bool inv) {
@@ -254,11 +214,6 @@ __device__ __forceinline__ void run_step(int s, const InstDev<float>& I, int pas
 }
 template <class T>
 __device__ __forceinline__ int step_radix(int s) { return sizeof(T) == 8 ? s : (s & 7) * (s >> 3); }
-// Steps of a pass: FP64 the divide's step is the last forward and the first inverse one, and the
-// inverse goes through the steps backwards; FP32 the inverse runs the plan from its start.
-template <class T>
-__host__ __device__ __forceinline__ int pass_steps(int n, int pass) { return pass != 2 ? n : (sizeof(T) == 8 ? 2 * n - 1 : 2 * n); }
-
 // Line group g of a pass. buf: two buffers of `half` values (the second unused by two steps or fewer).
 template <class T, bool XAXIS>
 __device__ __forceinline__ void fft_group(const InstDev<T>& I, int pass, int g, int LB, typename CxT<T>::type* buf, int half) {
@@ -267,7 +222,7 @@ __device__ __forceinline__ void fft_group(const InstDev<T>& I, int pass, int g, 
   const size_t NN = (size_t)N * N;
   Lines L;
   L.LB = LB;
-  L.pitch = N + N / 8 + 1;
+  L.pitch = x_pitch(N);
   L.x0 = L.y = 0;
   if (XAXIS) {
     L.base = (size_t)g * LB * N;
@@ -335,83 +290,27 @@ __global__ void __launch_bounds__(FFT_THREADS, fft_min_ctas<T>()) k_fft_plane(co
 
 // ---- host side -----------------------------------------------------------------------------
 
-constexpr int kRadix[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
-bool is_radix(int r) { return std::find(std::begin(kRadix), std::end(kRadix), r) != std::end(kRadix); }
-
-// Real operations per value of a radix-R step (the DFT of dft.cuh and its twiddles).
-double step_cost(int R) {
-  double c = 0;
-  switch (R) {
-    case 2: c = 2; break;
-    case 3: c = 4; break;
-    case 4: c = 4; break;
-    case 5: c = 7.2; break;
-    case 6: c = 6; break;
-    case 8: c = 6.5; break;
-    case 9: c = 9.8; break;
-    case 10: c = 9.2; break;
-    case 12: c = 8; break;
-    case 15: c = 11.2; break;
-    default: c = 10; break;
-  }
-  return c + 4.0 * (R - 1) / R;
-}
-
-// The steps for size N: fewest first (each boundary is a trip through shared memory), then fewest
-// operations; larger radices first.
-void best_steps(int N, int most, std::vector<int>& cur, std::vector<int>& best, double cost, double& best_cost) {
-  if (N == 1) {
-    if (best.empty() || cur.size() < best.size() || (cur.size() == best.size() && cost < best_cost)) {
-      best = cur;
-      best_cost = cost;
-    }
-    return;
-  }
-  if (!best.empty() && cur.size() >= best.size()) return;
-  for (int r : kRadix)
-    if (r <= most && N % r == 0) {
-      cur.push_back(r);
-      best_steps(N / r, r, cur, best, cost + step_cost(r), best_cost);
-      cur.pop_back();
-    }
-}
-std::vector<int> size_steps(int N) {
-  std::vector<int> cur, best;
-  double c = 0;
-  best_steps(N, 16, cur, best, 0, c);
-  return best;
-}
-// The default radix plan.
-std::vector<int> default_plan(int N) {
-  std::vector<int> p;
-  for (int r : {4, 2, 3, 5})
-    while (N % r == 0) { p.push_back(r); N /= r; }
-  return p;
-}
-bool is_pair(int r1, int r2) {
-#define X(A, B) if (r1 == A && r2 == B) return true;
-  TTSH_STAGE_PAIRS(X)
-#undef X
-  return false;
-}
-// The steps of a plan, as InstDev::step holds them.
-std::vector<int> plan_steps(float, int, const std::vector<int>& plan) {
+// The steps of a plan, as InstDev::step holds them: the best ones for N when the plan is the default
+// order, else (FP64) reversed for the reverse order or consecutive factors merged.
+std::vector<int> encode(const Steps& st, bool f64) {
   std::vector<int> s;
-  for (size_t k = 0; k < plan.size(); ++k) {
-    if (k + 1 < plan.size() && is_pair(plan[k], plan[k + 1])) {
-      s.push_back(pair_code(plan[k], plan[k + 1]));
-      ++k;
-    } else {
-      s.push_back(pair_code(plan[k], 1));
-    }
-  }
+  for (int i = 0; i < st.n; ++i) s.push_back(f64 ? st.a[i] : pair_code(st.a[i], st.b[i]));
   return s;
 }
+Radices radices(const std::vector<int>& plan) {
+  Radices p;
+  for (int r : plan) p.add(r);
+  return p;
+}
+bool is_default(int N, const std::vector<int>& plan) {
+  const Radices d = default_plan(N);
+  return plan == std::vector<int>(d.r, d.r + d.n);
+}
+std::vector<int> plan_steps(float, int, const std::vector<int>& plan) { return encode(stage_steps(radices(plan)), false); }
 std::vector<int> plan_steps(double, int N, const std::vector<int>& plan) {
-  std::vector<int> s = size_steps(N);
-  const std::vector<int> d = default_plan(N);
-  if (plan == d) return s;
-  if (plan == std::vector<int>(d.rbegin(), d.rend())) return std::vector<int>(s.rbegin(), s.rend());
+  std::vector<int> s = encode(default_steps<double>(N), true);
+  if (is_default(N, plan)) return s;
+  if (is_default(N, std::vector<int>(plan.rbegin(), plan.rend()))) return std::vector<int>(s.rbegin(), s.rend());
   s.clear();
   for (int r : plan) {
     if (!s.empty() && is_radix(s.back() * r)) s.back() *= r;
@@ -436,47 +335,8 @@ int pow2_lb(int N, size_t csize) {
   return lb;
 }
 
-// Default lines per CTA: the divisor of N whose steps, counted in whole warps per line, cost least,
-// among those that leave two CTAs' buffers on an SM (three for FP32) and whose rows along x are at
-// least 64 bytes where N allows. N = 100 in FP64: 25 lines (250 radix-10 butterflies in 8 warps; 4
-// lines, the largest power of two dividing 100, would fill 40 of 64 lanes).
 template <class T>
-int default_lb(int N) {
-  constexpr size_t csize = sizeof(typename CxT<T>::type);
-  const std::vector<int> st = plan_steps(T(0), N, default_plan(N));
-  const size_t room = (sizeof(T) == 4 ? 227 / 3 : 227 / 2) * 1024 - 1024;
-  int best = 0;
-  double cost = 0;
-  for (int lb = 1; lb <= std::min(N, 64); ++lb) {
-    if (N % lb != 0) continue;
-    if (lb > 1 && 2 * (size_t)half_values(N, lb) * csize > room) break;
-    double c = 0;
-    for (int s : st) {
-      const int r = sizeof(T) == 8 ? s : (s & 7) * (s >> 3);
-      const int warps = (lb * (N / r) + 31) / 32;
-      const int rounds = (warps + FFT_THREADS / 32 - 1) / (FFT_THREADS / 32);
-      // whole warps, and (a tenth of the weight) whole rounds of the CTA
-      c += (sizeof(T) == 8 ? step_cost(r) : 10.0) * r * (warps + 0.1 * (rounds * (FFT_THREADS / 32) - warps));
-    }
-    c /= lb;
-    if (lb * csize < 64) c *= 1.0 + 0.1 * (64.0 / (lb * csize) - 1);  // short rows along x
-    if (!best || c < cost * 0.999) {
-      best = lb;
-      cost = c;
-    }
-  }
-  return best;
-}
-
-template <class T>
-int threads_of(const Group<T>& g, int LB) {
-  int most = 0;
-  for (int s : plan_steps(T(0), g.N, default_plan(g.N))) {
-    const int r = sizeof(T) == 8 ? s : (s & 7) * (s >> 3);
-    most = std::max(most, LB * (g.N / r));
-  }
-  return std::min(FFT_THREADS, (most + 31) / 32 * 32);
-}
+int threads_of(const Group<T>& g, int LB) { return threads_for(default_steps<T>(g.N), g.N, LB); }
 
 inline void check_fft(const char* what) {
   cudaError_t e = cudaGetLastError();
@@ -495,6 +355,11 @@ void launch_one(const Group<T>& g, int pass, cudaStream_t st) {
 
 }  // namespace
 
+template <> bool fftplan_launch<float>(const Group<float>&, int, cudaStream_t);
+template <> bool fftplan_launch<double>(const Group<double>&, int, cudaStream_t);
+template <> void fftplan_prepare<float>(int);
+template <> void fftplan_prepare<double>(int);
+
 template <class T>
 void fft_steps(int N, const std::vector<int>& plan, int* step, int* nsteps) {
   const std::vector<int> s = plan_steps(T(0), N, plan);
@@ -504,10 +369,9 @@ void fft_steps(int N, const std::vector<int>& plan, int* step, int* nsteps) {
 
 template <class T>
 void launch_fft_plane(const Group<T>& g, int dir, cudaStream_t st) {
-  if (fftreg_plane_launch<T>(g, dir, st)) return;
+  if (fftreg_plane_launch<T>(g, dir, st) || fftplan_launch<T>(g, dir == 0 ? 0 : 4, st)) return;
   const int N = g.N, LB = fft_lines(g), half = half_values(N, LB), ng = N / LB;
-  int parts = 8;  // the cluster (8 CTAs at most is portable) splits a plane's line groups evenly
-  while (ng % parts != 0) --parts;
+  const int parts = cluster_parts(ng);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(N * parts, g.n);
   cfg.blockDim = dim3(threads_of(g, LB));
@@ -523,10 +387,37 @@ void launch_fft_plane(const Group<T>& g, int dir, cudaStream_t st) {
   if (e != cudaSuccess) throw std::runtime_error(std::string("fft (plane) launch: ") + cudaGetErrorString(e));
 }
 
+// The per-size kernels, in three translation units per type.
+#define X(NAME, T)                                            \
+  bool NAME##_launch(const Group<T>&, int, cudaStream_t);     \
+  bool NAME##_prepare(int);
+X(fftplan_f32_a, float) X(fftplan_f32_b, float) X(fftplan_f32_c, float)
+X(fftplan_f64_a, double) X(fftplan_f64_b, double) X(fftplan_f64_c, double)
+#undef X
+template <>
+bool fftplan_launch<float>(const Group<float>& g, int pass, cudaStream_t st) {
+  if (g.fft_kind != 2 || g.fft_lb != 0 || !g.fft_default) return false;
+  return fftplan_f32_a_launch(g, pass, st) || fftplan_f32_b_launch(g, pass, st) || fftplan_f32_c_launch(g, pass, st);
+}
+template <>
+bool fftplan_launch<double>(const Group<double>& g, int pass, cudaStream_t st) {
+  if (g.fft_kind != 2 || g.fft_lb != 0 || !g.fft_default) return false;
+  return fftplan_f64_a_launch(g, pass, st) || fftplan_f64_b_launch(g, pass, st) || fftplan_f64_c_launch(g, pass, st);
+}
+template <>
+void fftplan_prepare<float>(int N) {
+  if (!fftplan_f32_a_prepare(N) && !fftplan_f32_b_prepare(N)) fftplan_f32_c_prepare(N);
+}
+template <>
+void fftplan_prepare<double>(int N) {
+  if (!fftplan_f64_a_prepare(N) && !fftplan_f64_b_prepare(N)) fftplan_f64_c_prepare(N);
+}
+
 // One kernel serves every size, so its shared-memory limit is set once for all.
 template <class T>
 void fft_prepare(int N) {
   fftreg_prepare<T>(N);
+  fftplan_prepare<T>(N);
   for (const void* f : {(const void*)k_fft<T, true>, (const void*)k_fft<T, false>, (const void*)k_fft_plane<T>}) {
     const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFftSmem);
     if (e != cudaSuccess) throw std::runtime_error(std::string("fft smem attribute: ") + cudaGetErrorString(e));
@@ -560,7 +451,7 @@ int fft_lines(const Group<T>& g) {
 template <class T>
 void launch_fft_pass(const Group<T>& g, int pass, cudaStream_t st) {
   if (pass < 0 || pass > 4) throw std::runtime_error("bad fft pass");
-  if (fftreg_launch<T>(g, pass, st)) return;
+  if (fftreg_launch<T>(g, pass, st) || (pass == 2 && fftplan_launch<T>(g, pass, st))) return;
   launch_one<T>(g, pass, st);
 }
 

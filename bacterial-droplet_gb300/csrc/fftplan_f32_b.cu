@@ -1,0 +1,7 @@
+// fftplan_f32_b.cu — the per-size FFT kernels (fftplan_impl.cuh) of a third of the sizes, for float.
+#define TTSH_FFTPLAN_T float
+#include "fftplan_impl.cuh"
+
+namespace ttsh {
+TTSH_FFTPLAN_UNIT(fftplan_f32_b, float, TTSH_FFTPLAN_B)
+}  // namespace ttsh

@@ -17,6 +17,7 @@ struct Group {
   int fft_kind = 0;    // register-resident FFT kernels where the size has them, else Stockham: 0 one
                        // launch per axis pass, 2 x and y of a plane in one launch; 1: Stockham only
   int fft_lb = 0;      // Stockham lines per CTA (0: chosen by size, default_lb of fft.cu)
+  bool fft_default = true;  // the radix plan is the default order (4, 2, 3, 5)
   int fft_nsteps = 0;  // InstDev::nsteps of the group (0: not known, taken as three or more)
   int zc[3] = {0, 0, 0};     // z-planes per CTA of fused_rhs, fused_div, fused_correct
                              // (fused_default_zc); 0: the persistent grid (equal shares of the
@@ -69,6 +70,10 @@ template <class T> void launch_fft_plane(const Group<T>& g, int dir, cudaStream_
 // plan is the default order (4, 2, 3, 5) or its reverse, else consecutive factors of the plan merged.
 template <class T>
 void fft_steps(int N, const std::vector<int>& plan, int* step, int* nsteps);
+// The any-size FFT built per size (fftplan_impl.cuh), pass 2: z; 0: forward x + y of every plane; 4: inverse
+// y + x. False when the size has none or the group's configuration is not the default one.
+template <class T> bool fftplan_launch(const Group<T>& g, int pass, cudaStream_t st);
+template <class T> void fftplan_prepare(int N);
 // Sets the dynamic shared-memory limits of the FFT kernels for size N (call before capture).
 template <class T> void fft_prepare(int N);
 // Stockham lines per CTA: the explicit candidates for size N (largest first) and the one a group uses.

@@ -12,6 +12,10 @@ from test_gpu_cufft import cufft_projection, relerr
 pytestmark = pytest.mark.gpu
 
 
+def _factors(n):
+    return [p for p in range(2, n + 1) if n % p == 0 and all(p % q for q in range(2, p))]
+
+
 def projection(N, precision, steps=1, cfg=None):
     import ttsh
     st = random_state(N, seed=N + 3)
@@ -46,3 +50,28 @@ def test_launch_forms_give_the_same_bits(N, precision):
         got = projection(N, precision, 2, cfg)[0]
         for f in ("phi", "P", "u", "pv", "pp"):
             assert np.array_equal(got[f], want[f]), (cfg, f)
+
+
+# every size with kernels of its own (the products of 2, 3 and 5 up to 270 without a register kernel)
+PLAN_SIZES = [n for n in range(9, 271) if n not in (8, 16, 24, 32, 48, 64, 96, 128, 160, 192, 256)
+              and all(p in (2, 3, 5) for p in _factors(n))]
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_per_size_kernels_equal_the_any_size_kernel(precision):
+    """One solve of a random source by the kernels built for a size and by the kernel for any size (one
+    launch per axis): the same bits."""
+    import ttsh
+    rng = np.random.default_rng(0)
+    for N in PLAN_SIZES:
+        u, P = rng.standard_normal((2, 3, N, N, N)) * 0.01
+        phi = rng.random((N, N, N))
+        out = []
+        for kind in (2, 1):
+            with ttsh.Sim(ttsh.default_input(Nx=N, Ny=N, Nz=N), ttsh.default_ext(precision=precision, form=ttsh.FORM_PLAIN)) as s:
+                s.set_tuning(0, dict(s.tuning()[0], fft_kind=kind))
+                s.set_state(0, phi, P, u)
+                s.step(1)
+                out.append(s.get_state(0))
+        for f in ("pv", "pp", "u", "P"):
+            assert np.array_equal(out[0][f], out[1][f]), (N, f)

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fftplan.h"
 #include "fftreg.cuh"
 #include "kernels.h"
 
@@ -220,12 +221,14 @@ __device__ __forceinline__ void fft_lines(const InstDev<T>& I, int g, typename C
   }
 }
 
-// Minimum CTAs per SM. The FP32 z pass (forward, divide, inverse) trades a few
-// spilled registers for occupancy; measured at 256^3 (2 droplets): 4 CTAs 0.164 ms, 3 CTAs
-// 0.176 ms, 2 CTAs 0.196 ms per step. Other sizes keep the settings they were measured with.
+// Minimum CTAs per SM. The FP32 z pass (forward, divide, inverse) is bound by latency and issue and
+// gains from more resident warps as long as little is spilled. Measured, us per launch: 2 x 256^3 (when
+// its twiddles were read from global memory) 4 CTAs 164, 3 CTAs 176, 2 CTAs 196; 12 x 128^3 8 CTAs (64 registers) 83.5, 10 (48)
+// 89, no hint (80) 93; 8 x 96^3 14 CTAs 30.6, no hint 33.5; 4 x 192^3 7 CTAs 121, no hint 122.5; 512^3 3
+// CTAs 655, 4 (spills) 861; 6 x 160^3 no hint 148, 12 CTAs (spills) 215.
 template <class T, int N, int PASS>
 constexpr int fftr_min_blocks() {
-  return (sizeof(T) == 4 && PASS == 2) ? (N == 256 ? 4 : (N > 256 ? 3 : 1)) : 1;
+  return (sizeof(T) == 4 && PASS == 2) ? (N == 256 ? 4 : N > 256 ? 3 : N == 192 ? 7 : N == 128 ? 8 : N == 96 ? 14 : 1) : 1;
 }
 
 template <class T, int N1, int N2, int PASS>
@@ -241,10 +244,16 @@ __global__ void __launch_bounds__(lines_per_cta<N1 * N2>() * N2, fftr_min_blocks
 // every PC-th line group of the second axis. The plane's intermediate (N^2 complex values) is
 // written and read back a few microseconds apart, so it stays in L2 instead of making an HBM
 // round trip between two separate passes over the whole volume.
+// PC: as many CTAs as split the NG groups evenly, at most 8, except 4 for 8 and 16 groups. More CTAs
+// leave a smaller last wave of clusters and more of a plane in flight; at 16 groups a CTA's two turns
+// on each axis between cluster barriers are too few to cover them. Measured, us per launch of x+y and
+// y+x: one 160^3 droplet (10 groups) 45 / 60 with 2 parts, 32 / 38 with 5; one 96^3 (6) 16 / 21 with 2,
+// 12 / 12 with 6; 4 x 192^3 (12) 121 / 144 with 4, 118 / 144 with 6; 512^3 (32) 678 / 767 with 4, 624 / 686
+// with 8; one 256^3 (16) 76 / 78 with 4, 78 / 81 with 8.
 template <int N>
 constexpr int plane_parts() {
   constexpr int NG = N / lines_per_cta<N>();
-  return NG % 4 == 0 ? 4 : (NG % 2 == 0 ? 2 : (NG % 3 == 0 ? 3 : 1));
+  return NG == 8 || NG == 16 ? 4 : fftplan::cluster_parts(NG);
 }
 
 

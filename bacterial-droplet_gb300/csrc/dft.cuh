@@ -1,10 +1,10 @@
-// dft.cuh — small DFTs in registers, compile-time sizes 2 .. 16, for the FFT passes.
+// dft.cuh — small DFTs in registers, compile-time sizes 2 .. 40, for the FFT passes.
 //
 // Dft<R>::run(v): v[0..R) <- sum over n of v[n] exp(-2 pi i n k / R), natural order in and out, in place.
 // 2 and 4 are butterflies; 3 and 5 use the symmetry of their twiddles (the real and imaginary parts
 // of exp(2 pi i k / R) are even and odd in k), 12 and 36 real operations; 6, 10, 12, 15 are
-// prime-factor products (Good, 1958: the index maps below leave no twiddles between the factors);
-// 8, 9, 16 are two radix-2/4, 3 or 4 levels with the constant twiddles written out.
+// prime-factor products (Good, 1958: the index maps below leave no twiddles between the factors), and so
+// are 24 and 40; 8, 9, 16 are two radix-2/4, 3 or 4 levels with the constant twiddles written out.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -30,16 +30,19 @@ template <class C>
 __device__ __forceinline__ C mi(C a) { return mk<C>(a.y, -a.x); }  // -i a
 template <class C>
 __device__ __forceinline__ C axmi(C a, decltype(C::x) s, C b) { return axpy(a, s, mi(b)); }  // a + s (-i b)
-// a (1 - i) / sqrt 2 and a (-1 - i) / sqrt 2: the eighth roots of unity 1 and 3
+// 1 / sqrt 2 in FP64 from above and from below. As (HI, LO) the eighth roots of unity have magnitude 1 to
+// 1e-17; with the nearest value in both parts it would be 7e-17 off, the same way in every transform of
+// a solve.
+constexpr double R2_HI = 0.70710678118654757274, R2_LO = 0.70710678118654746172;
 template <class C>
-__device__ __forceinline__ C w8(C a) {
+__device__ __forceinline__ C w8(C a) {  // a exp(-2 pi i / 8)
   typedef decltype(C::x) T;
-  return mk<C>(T(0.70710678118654752440) * (a.x + a.y), T(0.70710678118654752440) * (a.y - a.x));
+  return mul(a, mk<C>(T(R2_HI), T(-R2_LO)));
 }
 template <class C>
-__device__ __forceinline__ C w83(C a) {
+__device__ __forceinline__ C w83(C a) {  // a exp(-6 pi i / 8)
   typedef decltype(C::x) T;
-  return mk<C>(T(0.70710678118654752440) * (a.y - a.x), T(-0.70710678118654752440) * (a.x + a.y));
+  return mul(a, mk<C>(T(-R2_LO), T(-R2_HI)));
 }
 
 template <int R>
@@ -204,6 +207,35 @@ struct Dft<16> {
       Dft<4>::run(t);
 #pragma unroll
       for (int j = 0; j < 4; ++j) v[k + 4 * j] = t[j];
+    }
+  }
+};
+
+template <> struct Dft<24> : DftPF<8, 3> {};
+template <> struct Dft<40> : DftPF<8, 5> {};
+// 32 = 2 x 16 (FP64): the even and odd inputs' DFTs, the odd ones times exp(-2 pi i k / 32)
+template <>
+struct Dft<32> {
+  static __device__ __forceinline__ void run(double2* v) {
+    constexpr double c[16] = {1, 0.98078528040323044913, 0.92387953251128675613, 0.83146961230254523708, R2_HI,
+                              0.55557023301960222474, 0.38268343236508977173, 0.19509032201612826785, 0,
+                              -0.19509032201612826785, -0.38268343236508977173, -0.55557023301960222474, -R2_LO,
+                              -0.83146961230254523708, -0.92387953251128675613, -0.98078528040323044913};  // cos(2 pi k / 32)
+    double2 e[16], o[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      e[k] = v[2 * k];
+      o[k] = v[2 * k + 1];
+    }
+    Dft<16>::run(e);
+    Dft<16>::run(o);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      // exp(-2 pi i k / 32) = cos - i sin, sin(2 pi k / 32) = cos(2 pi (k - 8) / 32)
+      const double sn = k == 4 ? R2_LO : (k == 12 ? R2_HI : c[k >= 8 ? k - 8 : 8 - k]);
+      const double2 x = k == 0 ? o[0] : (k == 8 ? mi(o[8]) : mul(o[k], mk<double2>(c[k], -sn)));
+      v[k] = add(e[k], x);
+      v[k + 16] = sub(e[k], x);
     }
   }
 };

@@ -85,16 +85,6 @@ struct Dft {
       v[2] = csub(a, c);
       v[1] = cadd(b, dd);
       v[3] = csub(b, dd);
-    } else if constexpr ((L == 3 || L == 5) && sizeof(v->x) == 8) {
-      dft::Dft<L>::run(v);
-      if (INV) {  // the inverse transform's output k is the forward one's -k
-#pragma unroll
-        for (int k = 1; 2 * k < L; ++k) {
-          const C t = v[k];
-          v[k] = v[L - k];
-          v[L - k] = t;
-        }
-      }
     } else if constexpr (L == 3 || L == 5) {
       C o[L];
 #pragma unroll

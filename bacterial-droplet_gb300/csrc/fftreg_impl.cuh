@@ -221,20 +221,122 @@ __device__ __forceinline__ void fft_lines(const InstDev<T>& I, int g, typename C
   }
 }
 
+// FP64: the same transforms with the small DFTs of dft.cuh, and the inverse as the forward transform
+// between conjugations (sign bits, no operations of the FP64 pipe, which bounds these kernels): 23.8
+// operations per value and 1-D transform instead of 24.3 at N = 256, 18 instead of 32 at 192 = 24 x 8
+// (prime-factor 24). (Letting the butterflies of the second DFT apply the four-step twiddles takes 21.3 at
+// 256, but rounds up to 40 % worse on the smooth pressures.) One solve, us: 192^3 2346 -> 2034, 160^3
+// 1455 -> 1338, 6 x 96^3 1503 -> 1341, 8 x 48^3 222 -> 206, with the register hints below 256^3 5386 -> 5075.
+template <int N1, int N2, int PASS>
+__device__ __forceinline__ void fft_lines64(const InstDev<double>& I, int g, double2* S) {
+  typedef double2 C;
+  constexpr int N = N1 * N2, LB = lines_per_cta<N>(), OW = N1 / N2;
+  constexpr int axis = (PASS == 0 || PASS == 4) ? 0 : ((PASS == 1 || PASS == 3) ? 1 : 2);
+  constexpr bool TW4C = axis != 0 || N2 <= 8;
+  C* __restrict__ W = I.W;
+  const C* tab = I.tw;
+  const int t = threadIdx.x;
+  const int l = axis == 0 ? t / N2 : t % LB, j = axis == 0 ? t % N2 : t / LB;
+  constexpr size_t stride = axis == 0 ? 1 : (axis == 1 ? N : (size_t)N * N);
+  int xl = 0, yl = 0;
+  size_t base;
+  if (axis == 0) {
+    base = ((size_t)g * LB + l) * N;
+  } else {
+    constexpr int ng = N / LB;
+    const int outer = g / ng;
+    xl = (g - outer * ng) * LB + l;
+    if (axis == 1) { base = (size_t)outer * N * N + xl; }
+    else { base = (size_t)outer * N + xl; yl = outer; }
+  }
+  auto sidx = [&](int k1, int n2) -> int {
+    return axis == 0 ? (l * (N1 * (N2 + 1)) + k1 * (N2 + 1) + n2) : ((k1 * N2 + n2) * LB + l);
+  };
+  auto tw = [&](int m) { return tw4<C, false, N, TW4C>(tab, m); };
+  if constexpr (PASS <= 2) {
+    C v[N1];
+#pragma unroll
+    for (int n1 = 0; n1 < N1; ++n1) v[n1] = W[base + (size_t)(N2 * n1 + j) * stride];
+    dft::Dft<N1>::run(v);
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) S[sidx(k1, j)] = v[k1];
+    __syncthreads();
+  }
+#pragma unroll
+  for (int o = 0; o < OW; ++o) {
+    const int k1 = j + N2 * o;
+    C u[N2];
+    if constexpr (PASS <= 2) {
+#pragma unroll
+      for (int n2 = 0; n2 < N2; ++n2) u[n2] = S[sidx(k1, n2)];
+#pragma unroll
+      for (int n2 = 1; n2 < N2; ++n2) u[n2] = dft::mul(u[n2], tw(n2 * k1));
+      dft::Dft<N2>::run(u);
+      if constexpr (PASS == 2) {
+        const Poisson<double> pm(I, xl, yl);
+#pragma unroll
+        for (int k2 = 0; k2 < N2; ++k2) u[k2] = dft::conj(pm(u[k2], I, k1 + N1 * k2));
+      } else {
+#pragma unroll
+        for (int k2 = 0; k2 < N2; ++k2) W[base + (size_t)(k1 + N1 * k2) * stride] = u[k2];
+      }
+    } else {
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2) u[k2] = dft::conj(W[base + (size_t)(k1 + N1 * k2) * stride]);
+    }
+    if constexpr (PASS >= 2) {
+      dft::Dft<N2>::run(u);
+#pragma unroll
+      for (int n2 = 0; n2 < N2; ++n2) S[sidx(k1, n2)] = u[n2];
+    }
+  }
+  if constexpr (PASS >= 2) {
+    __syncthreads();
+    C x[N1];
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) x[k1] = S[sidx(k1, j)];
+#pragma unroll
+    for (int k1 = 1; k1 < N1; ++k1) x[k1] = dft::mul(x[k1], tw(k1 * j));
+    dft::Dft<N1>::run(x);
+#pragma unroll
+    for (int n1 = 0; n1 < N1; ++n1) {
+      C o = dft::conj(x[n1]);
+      if constexpr (PASS == 4) o = scale_n3(o, I);
+      W[base + (size_t)(N2 * n1 + j) * stride] = o;
+    }
+  }
+}
+template <class T, int N1, int N2, int PASS>
+__device__ __forceinline__ void fft_group(const InstDev<T>& I, int g, typename CxT<T>::type* S) {
+  if constexpr (sizeof(T) == 8) fft_lines64<N1, N2, PASS>(I, g, S);
+  else fft_lines<T, N1, N2, PASS>(I, g, S);
+}
+
 // Minimum CTAs per SM. The FP32 z pass (forward, divide, inverse) is bound by latency and issue and
 // gains from more resident warps as long as little is spilled. Measured, us per launch: 2 x 256^3 (when
 // its twiddles were read from global memory) 4 CTAs 164, 3 CTAs 176, 2 CTAs 196; 12 x 128^3 8 CTAs (64 registers) 83.5, 10 (48)
 // 89, no hint (80) 93; 8 x 96^3 14 CTAs 30.6, no hint 33.5; 4 x 192^3 7 CTAs 121, no hint 122.5; 512^3 3
-// CTAs 655, 4 (spills) 861; 6 x 160^3 no hint 148, 12 CTAs (spills) 215.
+// CTAs 655, 4 (spills) 861; 6 x 160^3 no hint 148, 12 CTAs (spills) 215. In FP64 the hint puts two or
+// three CTAs on an SM, whose FP64 pipe idles while a lone CTA waits at a barrier (256^3: 1824 -> 1791).
 template <class T, int N, int PASS>
 constexpr int fftr_min_blocks() {
-  return (sizeof(T) == 4 && PASS == 2) ? (N == 256 ? 4 : N > 256 ? 3 : N == 192 ? 7 : N == 128 ? 8 : N == 96 ? 14 : 1) : 1;
+  if (PASS != 2) return 1;
+  if (sizeof(T) == 8) return N == 256 ? 2 : N == 192 ? 3 : 1;
+  return N == 256 ? 4 : N > 256 ? 3 : N == 192 ? 7 : N == 128 ? 8 : N == 96 ? 14 : 1;
+}
+// ... and of the plane kernels (0: no hint; at the other sizes it spills or gains nothing). us of x+y / y+x without and
+// with it: FP64 256^3 1821 / 1940 -> 1589 / 1695, 192^3 690 / 766 -> 623 / 667; FP32 2 x 256^3 160 / 166 ->
+// 158 / 160, 4 x 192^3 117 / 144 -> 118 / 131.
+template <class T, int N>
+constexpr int plane_min_blocks() {
+  if (sizeof(T) == 8) return N == 256 ? 2 : N == 192 ? 4 : 0;
+  return N == 256 ? 3 : N == 192 ? 6 : 0;
 }
 
 template <class T, int N1, int N2, int PASS>
 __global__ void __launch_bounds__(lines_per_cta<N1 * N2>() * N2, fftr_min_blocks<T, N1 * N2, PASS>()) k_fftr(const InstDev<T>* __restrict__ insts) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  fft_lines<T, N1, N2, PASS>(insts[blockIdx.y], blockIdx.x, reinterpret_cast<typename CxT<T>::type*>(smem_raw));
+  fft_group<T, N1, N2, PASS>(insts[blockIdx.y], blockIdx.x, reinterpret_cast<typename CxT<T>::type*>(smem_raw));
 }
 
 // Both in-plane axes of the z-planes, one plane per thread-block cluster of PC CTAs: DIR 0
@@ -277,30 +379,32 @@ __device__ __forceinline__ void plane_body(const InstDev<T>* __restrict__ insts)
   // groups z*NG .. of pass 1 / 3 (outer index z). __syncthreads between groups: the next group
   // reuses S.
   if constexpr (DIR == 0) {
-    for (int gg = part; gg < NG; gg += PC) { fft_lines<T, N1, N2, 0>(I, z * NG + gg, S); __syncthreads(); }
+    for (int gg = part; gg < NG; gg += PC) { fft_group<T, N1, N2, 0>(I, z * NG + gg, S); __syncthreads(); }
     cluster_sync_all();
-    for (int gg = part; gg < NG; gg += PC) { fft_lines<T, N1, N2, 1>(I, z * NG + gg, S); __syncthreads(); }
+    for (int gg = part; gg < NG; gg += PC) { fft_group<T, N1, N2, 1>(I, z * NG + gg, S); __syncthreads(); }
   } else {
-    for (int gg = part; gg < NG; gg += PC) { fft_lines<T, N1, N2, 3>(I, z * NG + gg, S); __syncthreads(); }
+    for (int gg = part; gg < NG; gg += PC) { fft_group<T, N1, N2, 3>(I, z * NG + gg, S); __syncthreads(); }
     cluster_sync_all();
-    for (int gg = part; gg < NG; gg += PC) { fft_lines<T, N1, N2, 4>(I, z * NG + gg, S); __syncthreads(); }
+    for (int gg = part; gg < NG; gg += PC) { fft_group<T, N1, N2, 4>(I, z * NG + gg, S); __syncthreads(); }
   }
 }
 
-// The kernels: without a register hint, and (FP32 at N = 256, measured 2 droplets: 0.158 / 0.160
-// ms per step against 0.160 / 0.166 ms without it) with 3 CTAs per SM; other sizes spill with it.
+// The kernels: without a register hint, and with one (plane_min_blocks).
 template <class T, int N1, int N2, int DIR>
 __global__ void __cluster_dims__(plane_parts<N1 * N2>(), 1, 1) __launch_bounds__(lines_per_cta<N1 * N2>() * N2)
     k_fftr_plane(const InstDev<T>* __restrict__ insts) {
   plane_body<T, N1, N2, DIR>(insts);
 }
 template <class T, int N1, int N2, int DIR>
-__global__ void __cluster_dims__(plane_parts<N1 * N2>(), 1, 1) __launch_bounds__(lines_per_cta<N1 * N2>() * N2, 3)
-    k_fftr_plane3(const InstDev<T>* __restrict__ insts) {
+__global__ void __cluster_dims__(plane_parts<N1 * N2>(), 1, 1)
+    __launch_bounds__(lines_per_cta<N1 * N2>() * N2, plane_min_blocks<T, N1 * N2>()) k_fftr_plane_hint(const InstDev<T>* __restrict__ insts) {
   plane_body<T, N1, N2, DIR>(insts);
 }
-template <class T, int N1, int N2>
-constexpr bool plane_hinted() { return sizeof(T) == 4 && N1 * N2 == 256; }
+template <class T, int N1, int N2, int DIR>
+constexpr auto plane_kernel() {
+  if constexpr (plane_min_blocks<T, N1 * N2>() > 0) return k_fftr_plane_hint<T, N1, N2, DIR>;
+  else return k_fftr_plane<T, N1, N2, DIR>;
+}
 
 // ---- the z pass with its input staged by the tensor memory accelerator (FP32) ----
 // Persistent CTAs: CTA b takes the z-line groups b, b + grid, ... of every droplet of the size
@@ -478,8 +582,7 @@ void launch_plane(const Group<T>& g, cudaStream_t st) {
   constexpr size_t smem = smem_bytes<T, N1, N2>(0) > smem_bytes<T, N1, N2>(1) ? smem_bytes<T, N1, N2>(0)
                                                                                 : smem_bytes<T, N1, N2>(1);
   const dim3 grid(N * plane_parts<N>(), g.n);
-  if constexpr (plane_hinted<T, N1, N2>()) k_fftr_plane3<T, N1, N2, DIR><<<grid, LB * N2, smem, st>>>(g.d_inst);
-  else k_fftr_plane<T, N1, N2, DIR><<<grid, LB * N2, smem, st>>>(g.d_inst);
+  plane_kernel<T, N1, N2, DIR>()<<<grid, LB * N2, smem, st>>>(g.d_inst);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("fft (register, plane) launch: ") + cudaGetErrorString(e));
 }
@@ -496,13 +599,8 @@ void prepare_size() {
   set((const void*)k_fftr<T, N1, N2, 3>, smem_bytes<T, N1, N2>(1));
   set((const void*)k_fftr<T, N1, N2, 4>, smem_bytes<T, N1, N2>(0));
   const size_t sp = smem_bytes<T, N1, N2>(0) > smem_bytes<T, N1, N2>(1) ? smem_bytes<T, N1, N2>(0) : smem_bytes<T, N1, N2>(1);
-  if constexpr (plane_hinted<T, N1, N2>()) {
-    set((const void*)k_fftr_plane3<T, N1, N2, 0>, sp);
-    set((const void*)k_fftr_plane3<T, N1, N2, 1>, sp);
-  } else {
-    set((const void*)k_fftr_plane<T, N1, N2, 0>, sp);
-    set((const void*)k_fftr_plane<T, N1, N2, 1>, sp);
-  }
+  set((const void*)plane_kernel<T, N1, N2, 0>(), sp);
+  set((const void*)plane_kernel<T, N1, N2, 1>(), sp);
 }
 
 template <class T, int N1, int N2>

@@ -43,7 +43,15 @@ int check() {
   return d < 4 * 1.2e-16 && f < 4 * 6e-8 ? 0 : 1;
 }
 
+template <int R>
+int check64() {
+  const double d = error<double2, R>();
+  std::printf("R=%d double %.2e\n", R, d);
+  return d < 5 * 1.2e-16 ? 0 : 1;
+}
+
 int main() {
+  if (check64<24>() + check64<32>() + check64<40>()) return 1;
   return check<2>() + check<3>() + check<4>() + check<5>() + check<6>() + check<8>() + check<9>() + check<10>() + check<12>() +
          check<15>() + check<16>();
 }

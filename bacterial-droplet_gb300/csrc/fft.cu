@@ -369,7 +369,8 @@ void fft_steps(int N, const std::vector<int>& plan, int* step, int* nsteps) {
 
 template <class T>
 void launch_fft_plane(const Group<T>& g, int dir, cudaStream_t st) {
-  if (fftreg_plane_launch<T>(g, dir, st) || fftplan_launch<T>(g, dir == 0 ? 0 : 4, st)) return;
+  // the per-size kernels come first: in FP64 the small sizes of the register kernels have them too
+  if (fftplan_launch<T>(g, dir == 0 ? 0 : 4, st) || fftreg_plane_launch<T>(g, dir, st)) return;
   const int N = g.N, LB = fft_lines(g), half = half_values(N, LB), ng = N / LB;
   const int parts = cluster_parts(ng);
   cudaLaunchConfig_t cfg{};
@@ -392,7 +393,7 @@ void launch_fft_plane(const Group<T>& g, int dir, cudaStream_t st) {
   bool NAME##_launch(const Group<T>&, int, cudaStream_t);     \
   bool NAME##_prepare(int);
 X(fftplan_f32_a, float) X(fftplan_f32_b, float) X(fftplan_f32_c, float)
-X(fftplan_f64_a, double) X(fftplan_f64_b, double) X(fftplan_f64_c, double)
+X(fftplan_f64_a, double) X(fftplan_f64_b, double) X(fftplan_f64_c, double) X(fftplan_f64_s, double)
 #undef X
 template <>
 bool fftplan_launch<float>(const Group<float>& g, int pass, cudaStream_t st) {
@@ -402,7 +403,7 @@ bool fftplan_launch<float>(const Group<float>& g, int pass, cudaStream_t st) {
 template <>
 bool fftplan_launch<double>(const Group<double>& g, int pass, cudaStream_t st) {
   if (g.fft_kind != 2 || g.fft_lb != 0 || !g.fft_default) return false;
-  return fftplan_f64_a_launch(g, pass, st) || fftplan_f64_b_launch(g, pass, st) || fftplan_f64_c_launch(g, pass, st);
+  return fftplan_f64_s_launch(g, pass, st) || fftplan_f64_a_launch(g, pass, st) || fftplan_f64_b_launch(g, pass, st) || fftplan_f64_c_launch(g, pass, st);
 }
 template <>
 void fftplan_prepare<float>(int N) {
@@ -410,6 +411,7 @@ void fftplan_prepare<float>(int N) {
 }
 template <>
 void fftplan_prepare<double>(int N) {
+  fftplan_f64_s_prepare(N);
   if (!fftplan_f64_a_prepare(N) && !fftplan_f64_b_prepare(N)) fftplan_f64_c_prepare(N);
 }
 
@@ -451,7 +453,7 @@ int fft_lines(const Group<T>& g) {
 template <class T>
 void launch_fft_pass(const Group<T>& g, int pass, cudaStream_t st) {
   if (pass < 0 || pass > 4) throw std::runtime_error("bad fft pass");
-  if (fftreg_launch<T>(g, pass, st) || (pass == 2 && fftplan_launch<T>(g, pass, st))) return;
+  if ((pass == 2 && fftplan_launch<T>(g, pass, st)) || fftreg_launch<T>(g, pass, st)) return;
   launch_one<T>(g, pass, st);
 }
 

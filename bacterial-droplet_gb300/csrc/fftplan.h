@@ -99,6 +99,25 @@ constexpr Steps default_steps(int N) {
   return best;
 }
 
+// The small sizes of the register kernels in FP64 (24, 32, 48). A grid of few warps is bound by the chain
+// of FP64 instructions of one thread, not by the pipe of the SM, so a step's butterflies go to as many
+// threads as it has (in the register kernels the threads of the first factor's DFTs take all of the
+// second's), 8 lines per CTA. The steps are the register kernels' factors in their order, and so are the
+// bits. One solve (three launches), us, register kernels / these: 32^3 48.5 / 42.6, 48^3 68.4 / 59.4, 24^3
+// 59.9 / 50.1; where the pipe is full they are level (8 x 48^3 206 / 208, 24 x 32^3 187 / 183).
+constexpr Steps small_steps(int N) {
+  const int first = N % 3 == 0 ? 12 : 8;
+  Steps s;
+  s.add(first, 1);
+  s.add(N / first, 1);
+  return s;
+}
+constexpr int small_lb(int N) {
+  int lb = 8;
+  while (N % lb != 0) --lb;
+  return lb;
+}
+
 constexpr int kThreads = 256;  // most threads of a CTA
 // Lines along x lie one after another in shared memory, elements spread by one in eight.
 constexpr int x_pitch(int N) { return N + N / 8 + 1; }

@@ -20,35 +20,40 @@
 namespace ttsh {
 namespace fftplan {
 
-template <class T, int N>
+template <class T, int N, bool SMALL>
 struct Plan {
-  static constexpr Steps S = default_steps<T>(N);
-  static constexpr int LB = default_lb<T>(N), NG = N / LB, PC = cluster_parts(NG), THREADS = threads_for(S, N, LB);
+  static constexpr Steps S = SMALL ? small_steps(N) : default_steps<T>(N);
+  static constexpr int LB = SMALL ? small_lb(N) : default_lb<T>(N), NG = N / LB, PC = cluster_parts(NG), THREADS = threads_for(S, N, LB);
   static constexpr int HALF = LB * x_pitch(N);  // values of one buffer
   static_assert(N % LB == 0 && 2 * HALF * 2 * sizeof(T) <= 227 * 1024, "lines per CTA");
   static constexpr int ops(int pass) { return pass_steps<T>(S.n, pass); }
   static constexpr size_t smem(int pass) {
     return (size_t)(ops(pass) < 2 ? 0 : (ops(pass) == 2 ? 1 : 2)) * HALF * sizeof(typename CxT<T>::type);
   }
-  // operation q of a pass: its step, and the product of the radices before it
-  static constexpr int step_of(int q) { return q < S.n ? q : (sizeof(T) == 8 ? 2 * S.n - 2 - q : q - S.n); }
-  static constexpr int before(int q) {
+  // operation q of a pass: its step, and the product of the radices before it. The inverse x and y
+  // transforms of a small size go through the steps backwards, as the register kernels do.
+  static constexpr bool back(int q, int pass) { return sizeof(T) == 8 && (q >= S.n || (SMALL && pass >= 3)); }
+  static constexpr int step_of(int q, int pass) {
+    if (pass != 2) return back(q, pass) ? S.n - 1 - q : q;
+    return q < S.n ? q : (back(q, pass) ? 2 * S.n - 2 - q : q - S.n);
+  }
+  static constexpr int before(int q, int pass) {
     int p = 1;
-    if (q < S.n || sizeof(T) == 4) {
-      for (int i = 0; i < step_of(q); ++i) p *= S.radix(i);
+    if (back(q, pass)) {
+      for (int i = S.n - 1; i > step_of(q, pass); --i) p *= S.radix(i);
     } else {
-      for (int i = S.n - 1; i > step_of(q); --i) p *= S.radix(i);
+      for (int i = 0; i < step_of(q, pass); ++i) p *= S.radix(i);
     }
     return p;
   }
 };
 
 // Operation Q of a pass and the ones after it, on the lines whose first element is at W + base.
-template <class T, int N, int PASS, int Q>
+template <class T, int N, bool SMALL, int PASS, int Q>
 __device__ __forceinline__ void run_ops(const InstDev<T>& I, size_t base, int x0, int y, typename CxT<T>::type* buf) {
   typedef typename CxT<T>::type C;
-  typedef Plan<T, N> P;
-  constexpr int OPS = P::ops(PASS), IDX = P::step_of(Q), A = P::S.a[IDX], B = P::S.b[IDX], R = A * B, M = N / R, NS = P::before(Q);
+  typedef Plan<T, N, SMALL> P;
+  constexpr int OPS = P::ops(PASS), IDX = P::step_of(Q, PASS), A = P::S.a[IDX], B = P::S.b[IDX], R = A * B, M = N / R, NS = P::before(Q, PASS);
   constexpr bool XAXIS = PASS == 0 || PASS == 4, FIRST = Q == 0, LAST = Q == OPS - 1, DIVIDE = PASS == 2 && Q == P::S.n - 1;
   constexpr bool INV = PASS >= 3 || Q >= P::S.n;
   constexpr size_t STRIDE = XAXIS ? 1 : (PASS == 2 ? (size_t)N * N : N), LSTRIDE = XAXIS ? N : 1;
@@ -138,19 +143,19 @@ __device__ __forceinline__ void run_ops(const InstDev<T>& I, size_t base, int x0
   }
   if constexpr (!LAST) {
     __syncthreads();
-    run_ops<T, N, PASS, Q + 1>(I, base, x0, y, buf);
+    run_ops<T, N, SMALL, PASS, Q + 1>(I, base, x0, y, buf);
   }
 }
 
 // Line group g of a pass.
-template <class T, int N, int PASS>
+template <class T, int N, bool SMALL, int PASS>
 __device__ __forceinline__ void run_group(const InstDev<T>& I, int g, typename CxT<T>::type* buf) {
-  typedef Plan<T, N> P;
+  typedef Plan<T, N, SMALL> P;
   if constexpr (PASS == 0 || PASS == 4) {
-    run_ops<T, N, PASS, 0>(I, (size_t)g * P::LB * N, 0, 0, buf);
+    run_ops<T, N, SMALL, PASS, 0>(I, (size_t)g * P::LB * N, 0, 0, buf);
   } else {
     const int outer = g / P::NG, x0 = (g - outer * P::NG) * P::LB;
-    run_ops<T, N, PASS, 0>(I, (size_t)outer * (PASS == 2 ? N : N * N) + x0, x0, outer, buf);
+    run_ops<T, N, SMALL, PASS, 0>(I, (size_t)outer * (PASS == 2 ? N : N * N) + x0, x0, outer, buf);
   }
 }
 
@@ -158,40 +163,40 @@ template <class T>
 constexpr int min_ctas() { return sizeof(T) == 4 ? 3 : 2; }
 
 // z lines
-template <class T, int N>
-__global__ void __launch_bounds__(Plan<T, N>::THREADS, min_ctas<T>()) k_plan_z(const InstDev<T>* __restrict__ insts) {
+template <class T, int N, bool SMALL>
+__global__ void __launch_bounds__(Plan<T, N, SMALL>::THREADS, min_ctas<T>()) k_plan_z(const InstDev<T>* __restrict__ insts) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  run_group<T, N, 2>(insts[blockIdx.y], blockIdx.x, reinterpret_cast<typename CxT<T>::type*>(smem_raw));
+  run_group<T, N, SMALL, 2>(insts[blockIdx.y], blockIdx.x, reinterpret_cast<typename CxT<T>::type*>(smem_raw));
 }
 // Both in-plane axes of a z-plane, one cluster per plane (as k_fft_plane): FIRST pass, then SECOND.
-template <class T, int N, int FIRST, int SECOND>
-__global__ void __cluster_dims__(Plan<T, N>::PC, 1, 1) __launch_bounds__(Plan<T, N>::THREADS, min_ctas<T>())
+template <class T, int N, bool SMALL, int FIRST, int SECOND>
+__global__ void __cluster_dims__(Plan<T, N, SMALL>::PC, 1, 1) __launch_bounds__(Plan<T, N, SMALL>::THREADS, min_ctas<T>())
     k_plan_plane(const InstDev<T>* __restrict__ insts) {
-  typedef Plan<T, N> P;
+  typedef Plan<T, N, SMALL> P;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto* buf = reinterpret_cast<typename CxT<T>::type*>(smem_raw);
   const InstDev<T>& I = insts[blockIdx.y];
   const int z = blockIdx.x / P::PC, part = blockIdx.x % P::PC;
 #pragma unroll 1
   for (int gg = part; gg < P::NG; gg += P::PC) {
-    run_group<T, N, FIRST>(I, z * P::NG + gg, buf);
+    run_group<T, N, SMALL, FIRST>(I, z * P::NG + gg, buf);
     __syncthreads();  // the next group reuses the buffers
   }
   asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 #pragma unroll 1
   for (int gg = part; gg < P::NG; gg += P::PC) {
-    run_group<T, N, SECOND>(I, z * P::NG + gg, buf);
+    run_group<T, N, SMALL, SECOND>(I, z * P::NG + gg, buf);
     __syncthreads();
   }
 }
 
-template <class T, int N>
+template <class T, int N, bool SMALL>
 void prepare_one() {
-  typedef Plan<T, N> P;
-  const std::pair<const void*, size_t> k[] = {{(const void*)k_plan_z<T, N>, P::smem(2)},
-                                              {(const void*)k_plan_plane<T, N, 0, 1>, P::smem(0)},
-                                              {(const void*)k_plan_plane<T, N, 3, 4>, P::smem(3)}};
+  typedef Plan<T, N, SMALL> P;
+  const std::pair<const void*, size_t> k[] = {{(const void*)k_plan_z<T, N, SMALL>, P::smem(2)},
+                                              {(const void*)k_plan_plane<T, N, SMALL, 0, 1>, P::smem(0)},
+                                              {(const void*)k_plan_plane<T, N, SMALL, 3, 4>, P::smem(3)}};
   for (const auto& f : k) {
     const cudaError_t e = cudaFuncSetAttribute(f.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.second);
     if (e != cudaSuccess) throw std::runtime_error(std::string("fft (plan) smem attribute: ") + cudaGetErrorString(e));
@@ -199,12 +204,12 @@ void prepare_one() {
 }
 
 // pass 2: the z lines; 0: forward x + y of every plane; 4: inverse y + x
-template <class T, int N>
+template <class T, int N, bool SMALL>
 void launch_size(const Group<T>& g, int pass, cudaStream_t st) {
-  typedef Plan<T, N> P;
-  if (pass == 2) k_plan_z<T, N><<<dim3(N * P::NG, g.n), P::THREADS, P::smem(2), st>>>(g.d_inst);
-  else if (pass == 0) k_plan_plane<T, N, 0, 1><<<dim3(N * P::PC, g.n), P::THREADS, P::smem(0), st>>>(g.d_inst);
-  else k_plan_plane<T, N, 3, 4><<<dim3(N * P::PC, g.n), P::THREADS, P::smem(3), st>>>(g.d_inst);
+  typedef Plan<T, N, SMALL> P;
+  if (pass == 2) k_plan_z<T, N, SMALL><<<dim3(N * P::NG, g.n), P::THREADS, P::smem(2), st>>>(g.d_inst);
+  else if (pass == 0) k_plan_plane<T, N, SMALL, 0, 1><<<dim3(N * P::PC, g.n), P::THREADS, P::smem(0), st>>>(g.d_inst);
+  else k_plan_plane<T, N, SMALL, 3, 4><<<dim3(N * P::PC, g.n), P::THREADS, P::smem(3), st>>>(g.d_inst);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("fft (plan) launch: ") + cudaGetErrorString(e));
 }
@@ -226,13 +231,18 @@ void launch_size(const Group<T>& g, int pass, cudaStream_t st) {
       default: return false;                                                  \
     }                                                                         \
   }
-#define TTSH_FFTPLAN_LAUNCH(n) case n: fftplan::launch_size<TTSH_FFTPLAN_T, n>(g, pass, st); return true;
-#define TTSH_FFTPLAN_PREPARE(n) case n: fftplan::prepare_one<TTSH_FFTPLAN_T, n>(); return true;
+#ifndef TTSH_FFTPLAN_SMALL
+#define TTSH_FFTPLAN_SMALL false
+#endif
+#define TTSH_FFTPLAN_LAUNCH(n) case n: fftplan::launch_size<TTSH_FFTPLAN_T, n, TTSH_FFTPLAN_SMALL>(g, pass, st); return true;
+#define TTSH_FFTPLAN_PREPARE(n) case n: fftplan::prepare_one<TTSH_FFTPLAN_T, n, TTSH_FFTPLAN_SMALL>(); return true;
 
 // The products of 2, 3 and 5 up to 500 without a register kernel (fftreg_impl.cuh).
 #define TTSH_FFTPLAN_A(X) X(9) X(10) X(12) X(15) X(18) X(20) X(25) X(27) X(30) X(36) X(40) X(45) X(50) X(54) X(60) X(72)
 #define TTSH_FFTPLAN_B(X) X(75) X(80) X(81) X(90) X(100) X(108) X(120) X(125) X(135) X(144) X(150) X(162) X(180) X(200) X(216)
 #define TTSH_FFTPLAN_C(X) \
   X(225) X(240) X(243) X(250) X(270) X(288) X(300) X(320) X(324) X(360) X(375) X(384) X(400) X(405) X(432) X(450) X(480) X(486) X(500)
+// The small sizes of the register kernels in FP64 (small_steps): 8 and 16 gain nothing.
+#define TTSH_FFTPLAN_S(X) X(24) X(32) X(48)
 
 }  // namespace ttsh

@@ -18,7 +18,7 @@ OBJDIR = os.path.join(LIBDIR, "obj")
 LIB = os.path.join(LIBDIR, "libttsh.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = ["api.cu", "plain.cu", "fft.cu", "fftplan_f32_a.cu", "fftplan_f32_b.cu", "fftplan_f32_c.cu",
-           "fftplan_f64_a.cu", "fftplan_f64_b.cu", "fftplan_f64_c.cu", "fftreg_f32.cu", "fftreg_f64.cu", "fused.cu", "io.cpp", "noalloc.cu", "plain64.cu", "post.cu"]
+           "fftplan_f64_a.cu", "fftplan_f64_b.cu", "fftplan_f64_c.cu", "fftplan_f64_s.cu", "fftreg_f32.cu", "fftreg_f64.cu", "fused.cu", "io.cpp", "noalloc.cu", "plain64.cu", "post.cu"]
 
 
 def nvcc() -> str:

@@ -57,10 +57,14 @@ KERNEL_WORDS = {
     "fused_div": 11,        # reads u*, P* and their compensations (6 + 3); writes the packed source W (2)
     "fused_correct": 18.5,  # reads u*, P*, compensations, the packed pressure (6 + 3 + 2); writes u, P and
                             # the compensation of u (6 + 1.5)
-    "stage1": 17, "stage2": 27, "div": 8, "correct": 14,  # plain form
+    "stage1": 17, "stage2": 27, "div": 8, "correct": 14,  # plain form (FP64: KERNEL_WORDS_F64)
     "fft_x_fwd": 4, "fft_y_fwd": 4, "fft_z_poisson": 4, "fft_y_inv": 4, "fft_x_inv": 4,
     "fft_xy_fwd": 4, "fft_yx_inv": 4,  # x and y of a plane in one launch: W read and written once
 }
+
+# FP64 plain form: stage1 also takes the pointwise parts of the step (reads phi, P, u; writes mu_0, mu, sigma
+# and those parts), stage2 adds them (reads the 20 words of stage1, phi, P, u; writes phi', u*, P*)
+KERNEL_WORDS_F64 = {"stage1": 27, "stage2": 34}
 
 # DRAM bytes per site of the dominant FP32 kernels, dram__bytes_read.sum + dram__bytes_write.sum
 # of one ncu capture of the default configuration on a 256^3 droplet (--clock-control none); a
@@ -430,7 +434,8 @@ def main():
     peak, peak_kind = measured_peak_hbm()
     dom = max(prof.items(), key=lambda kv: kv[1][0])
     dom_name, (dom_ms, dom_launches) = dom
-    dom_bytes = KERNEL_WORDS.get(dom_name, 0) * wbytes * sites
+    words = KERNEL_WORDS if args.precision == 32 else {**KERNEL_WORDS, **KERNEL_WORDS_F64}
+    dom_bytes = words.get(dom_name, 0) * wbytes * sites
     achieved = dom_bytes / (dom_ms / 1e3) / 1e9 if dom_ms > 0 else 0.0
     traffic = None
     if args.precision == 32 and dom_name in TRAFFIC_BYTES_PER_SITE_F32:

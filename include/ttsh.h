@@ -239,9 +239,9 @@ int ttsh_struct_size(int which);
 typedef struct {
   int N;           /* droplet size of the group */
   int n;           /* droplets in the group */
-  int fft_kind;    /* register-resident kernels where the size has them: 0 one launch per axis
-                      pass, 2 x and y of each plane in one launch; 1 Stockham */
-  int fft_lb;      /* Stockham lines per CTA; 0 = the largest that fits */
+  int fft_kind;    /* register-resident kernels where the size has them, else the Stockham ones: 0 one
+                      launch per axis pass, 2 x and y of each plane in one launch; 1 Stockham per axis */
+  int fft_lb;      /* Stockham lines per CTA; 0 = chosen by the size */
   int nstages;     /* Stockham radix plan: radix[0..nstages-1], each 2, 3, 4 or 5, product N */
   int radix[16];
   int zc[3];       /* z-planes per CTA of fused_rhs, fused_div, fused_correct (fused form);

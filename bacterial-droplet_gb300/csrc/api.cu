@@ -400,7 +400,7 @@ void build_engine(ttsh_sim* s, Engine<T>& E) {
     G.N = s->inst[E.members[g][0]].N;
     G.fft_nsteps = E.h[E.members[g][0]].nsteps;
     G.d_err = s->d_err;
-    if (s->fused) fused_default_zc(G.N, G.n, G.zc);
+    if (s->fused) fused_default_zc(G.N, G.n, E.members.size() == 1, G.zc);
     // FP32, on request (TTSH_ZTMA=1): the z pass with its input staged by the tensor memory
     // accelerator where the size has it; by default the z pass loads its input directly (faster
     // since its twiddles come from constant memory)

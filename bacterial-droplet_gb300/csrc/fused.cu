@@ -991,8 +991,15 @@ static int persistent_grid(const void* kernel, int threads, size_t smem, long lo
   return (int)std::min<long long>(*cache, planes);
 }
 
-// Default schedules of a group of n droplets of size N. fused_rhs: the persistent grid (within 3 %
-// of the best chunk at every group size measured). fused_div and fused_correct: chunks of z-planes,
+// Default schedules of a group of n droplets of size N. fused_rhs: the persistent grid, or, where the group
+// is the batch's only one (alone; the branches of several share the device: 2 x 96^3 .. 192^3 2466 us per
+// step with persistent grids, 2520 with 96^3 in chunks) and one wave of equal chunks has few more planes per CTA than the persistent grid's share, these: a CTA of the
+// persistent grid whose share crosses tiles loads four halo planes again. Measured, us per launch,
+// persistent / chunks (planes per chunk - share): one 96^3 66 / 57 (0.6), one 160^3 219 / 209 (1.4), 2 x 64^3
+// 47 / 43 (1.3), 2 x 96^3 108 / 102 (1.3), 4 x 96^3 192 / 188 (2.5), 3 x 160^3 605 / 593 (2.1), 18 x 64^3 244 /
+// 244 (3.4), 8 x 96^3 355 / 360 (5.1), one 128^3 121 / 131 (5.1); with shares of 1 .. 6 planes the rest of
+// the wave decides (one 64^3, 3.4 planes: 28.5 / 29.3), up to 1 both give every CTA one plane (one 32^3 14.6 /
+// 13.9). fused_div and fused_correct: chunks of z-planes,
 // long enough to amortise the stencils' two halo planes and the ring's first copies, but short
 // enough that one wave of CTAs covers every SM: the planes are cut into as many chunks as one wave
 // holds (3 or 2 CTAs per SM), at most 40 (fused_div) or 20 (fused_correct) planes each. Measured, us
@@ -1000,7 +1007,7 @@ static int persistent_grid(const void* kernel, int threads, size_t smem, long lo
 // 15 and 64 -> 11; 2 x 96^3 86 -> 35 and 75 -> 29; 12 x 128^3 (the caps; longer chunks leave a partial
 // last wave, shorter ones re-read halos: 8 planes 336 / 315, 64 planes 325 / 335) 325 -> 309 and
 // 335 -> 310; 2 x 256^3 378 -> 376 and 430 -> 409.
-void fused_default_zc(int N, int n, int zc[3]) {
+void fused_default_zc(int N, int n, bool alone, int zc[3]) {
   int dev = 0, sms = 0;
   check(cudaGetDevice(&dev), "fused: device");
   check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "fused: SM count");
@@ -1013,7 +1020,9 @@ void fused_default_zc(int N, int n, int zc[3]) {
     if ((long long)chunks * n > 65535) return N;  // the grid's limit: very many small droplets
     return (N + chunks - 1) / chunks;             // equal chunks
   };
-  zc[0] = 0;
+  const int z = planes(2, TYR, N);
+  const double places = 2.0 * sms, columns = (double)n * (N / TX) * (N / TYR), share = N * columns / places;
+  zc[0] = alone && columns <= places && z <= share + 3 && (share <= 1 || share >= 6) ? z : 0;
   zc[1] = planes(3, TYD, 40);
   zc[2] = planes(2, TY, 20);
 }

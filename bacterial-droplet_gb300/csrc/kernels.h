@@ -98,7 +98,7 @@ void launch_fused_div(const Group<float>& g, int par, cudaStream_t st);
 void launch_fused_correct(const Group<float>& g, int par, cudaStream_t st);
 bool fused_supported(int N);
 // The schedules (Group::zc) a group of n droplets of size N starts with.
-void fused_default_zc(int N, int n, int zc[3]);
+void fused_default_zc(int N, int n, bool alone, int zc[3]);
 // Sets the fused kernels' dynamic shared-memory limits (call before capture).
 void fused_prepare();
 

@@ -265,43 +265,46 @@ void build_engine(ttsh_sim* s, Engine<T>& E) {
     E.loc[i] = (int)E.members[E.grp[i]].size();
     E.members[E.grp[i]].push_back(i);
   }
-  // per-N tables
-  std::map<int, InstDev<T>> tab;
+  // Twiddles per N, wavenumber tables per (N, h): droplets of one size may differ in h.
+  auto upload = [&](const void* src, size_t bytes) {
+    void* d = nullptr;
+    CK(cudaMalloc(&d, bytes));
+    s->tables.push_back(d);
+    CK(cudaMemcpy(d, src, bytes, cudaMemcpyHostToDevice));
+    return d;
+  };
+  std::map<std::pair<int, double>, InstDev<T>> tab;
   for (auto& kv : by_n) {
     const int N = kv.first;
-    const double h = s->inst[E.members[kv.second][0]].in.h;
     std::vector<C> tw(N);
-    std::vector<double> kval(N);
-    std::vector<T> k2t(N), St(N), Ct(N);
     for (int k = 0; k < N; ++k) {
       const double a = -2.0 * kPi * (double)k / (double)N;
       tw[k].x = (T)std::cos(a);
       tw[k].y = (T)std::sin(a);
-      // initPoissonSolver (TTSH3D.cu:1093-1117)
-      double kk = 2 * kPi * k / (N * h + 0.0);
-      if (k >= N / 2) kk = 2 * kPi * (k - N) / (N * h + 0.0);
-      kval[k] = kk;
-      k2t[k] = (T)(kk * kk);
-      St[k] = (T)(std::sin(kk * h) / h);
-      Ct[k] = (T)((2.0 + std::cos(kk * h)) / 3.0);
     }
-    size_t bytes = align256(N * sizeof(C)) + align256(N * sizeof(double)) + 3 * align256(N * sizeof(T));
-    char* d = nullptr;
-    CK(cudaMalloc(&d, bytes));
-    s->tables.push_back(d);
-    InstDev<T> t{};
-    size_t off = 0;
-    t.tw = reinterpret_cast<C*>(d + off); CK(cudaMemcpy(d + off, tw.data(), N * sizeof(C), cudaMemcpyHostToDevice));
-    off += align256(N * sizeof(C));
-    t.kval = reinterpret_cast<double*>(d + off);
-    CK(cudaMemcpy(d + off, kval.data(), N * sizeof(double), cudaMemcpyHostToDevice));
-    off += align256(N * sizeof(double));
-    t.k2t = reinterpret_cast<T*>(d + off); CK(cudaMemcpy(d + off, k2t.data(), N * sizeof(T), cudaMemcpyHostToDevice));
-    off += align256(N * sizeof(T));
-    t.St = reinterpret_cast<T*>(d + off); CK(cudaMemcpy(d + off, St.data(), N * sizeof(T), cudaMemcpyHostToDevice));
-    off += align256(N * sizeof(T));
-    t.Ct = reinterpret_cast<T*>(d + off); CK(cudaMemcpy(d + off, Ct.data(), N * sizeof(T), cudaMemcpyHostToDevice));
-    tab[N] = t;
+    const C* d_tw = static_cast<const C*>(upload(tw.data(), N * sizeof(C)));
+    for (int i : E.members[kv.second]) {
+      const double h = s->inst[i].in.h;
+      if (tab.count({N, h})) continue;
+      std::vector<double> kval(N);
+      std::vector<T> t3(3 * N);  // k^2, sin(k h)/h, (2 + cos(k h))/3
+      for (int k = 0; k < N; ++k) {
+        // initPoissonSolver (TTSH3D.cu:1093-1117)
+        double kk = 2 * kPi * k / (N * h + 0.0);
+        if (k >= N / 2) kk = 2 * kPi * (k - N) / (N * h + 0.0);
+        kval[k] = kk;
+        t3[k] = (T)(kk * kk);
+        t3[N + k] = (T)(std::sin(kk * h) / h);
+        t3[2 * N + k] = (T)((2.0 + std::cos(kk * h)) / 3.0);
+      }
+      InstDev<T> t{};
+      t.tw = d_tw;
+      t.kval = static_cast<const double*>(upload(kval.data(), N * sizeof(double)));
+      t.k2t = static_cast<const T*>(upload(t3.data(), 3 * N * sizeof(T)));
+      t.St = t.k2t + N;
+      t.Ct = t.St + N;
+      tab[{N, h}] = t;
+    }
     fft_prepare<T>(N);
     if (sizeof(T) == 8) plain64_prepare(N);
     else if (!s->fused) plain32_prepare();
@@ -325,7 +328,7 @@ void build_engine(ttsh_sim* s, Engine<T>& E) {
     ih.arena = d;
     CK(cudaMemset(d, 0, bytes));
     InstDev<T>& I = E.h[i];
-    I = tab[N];
+    I = tab[{N, ih.in.h}];
     I.N = N;
     I.stale = (ih.ext.quirks & TTSH_QUIRK_STALE_HALO) ? 1 : 0;
     I.k2mode = ih.ext.k2_mode;

@@ -743,13 +743,20 @@ void tune_group(ttsh_sim* s, Engine<T>& E, size_t gi, ttsh_tuning* out) {
     auto fft = [&]() {
       enqueue_fft(G, st, [](int, auto&& f) { f(); });
     };
+    // the configuration the group runs with is the first candidate: only a faster one replaces it
     struct Cand { int kind, lb; std::vector<int> radix; };
-    std::vector<Cand> cands;
+    const InstDev<T>& cur = E.h[E.members[gi][0]];
+    std::vector<Cand> cands = {{G.fft_kind, G.fft_lb, std::vector<int>(cur.radix, cur.radix + cur.nstages)}};
+    auto add = [&](int kind, int lb, const std::vector<int>& radix) {
+      for (const Cand& c : cands)
+        if (c.kind == kind && c.lb == lb && c.radix == radix) return;
+      cands.push_back({kind, lb, radix});
+    };
     const std::vector<std::vector<int>> orders = radix_orders(G.N);
-    cands.push_back({2, 0, orders[0]});
-    cands.push_back({0, 0, orders[0]});
+    add(2, 0, orders[0]);
+    add(0, 0, orders[0]);
     for (int lb : fft_lb_candidates<T>(G.N))
-      for (const auto& o : orders) cands.push_back({1, lb, o});
+      for (const auto& o : orders) add(1, lb, o);
     double best = 1e30;
     Cand pick = cands[0];
     for (const Cand& c : cands) {
@@ -764,13 +771,17 @@ void tune_group(ttsh_sim* s, Engine<T>& E, size_t gi, ttsh_tuning* out) {
     set_radix(s, E, gi, pick.radix);
     double ms[4] = {best, 0, 0, 0};
     if (s->fused) {
-      // z-planes per CTA; 0: the persistent grid (equal shares of the group's sites per CTA)
-      const int zcs[] = {0, 8, 16, 32, 64, 128, 256};
+      // z-planes per CTA: the group's own, the default, the persistent grid (0: equal shares of the
+      // group's sites per CTA), and powers of two
+      int dflt[3];
+      fused_default_zc(G.N, G.n, E.groups.size() == 1, dflt);
       for (int k = 0; k < 3; ++k) {
         double bk_t = 1e30;
         int bk_z = G.zc[k];
+        std::vector<int> zcs = {G.zc[k]};
+        for (int z : {dflt[k], 0, 8, 16, 32, 64, 128, 256})
+          if (std::find(zcs.begin(), zcs.end(), z) == zcs.end() && z <= G.N) zcs.push_back(z);
         for (int z : zcs) {
-          if (z > G.N && z != zcs[1]) continue;
           if (z > 0 && (long)((G.N + z - 1) / z) * G.n > 65535) continue;
           G.zc[k] = z;
           const double t = time_graph(st, reps, [] {}, [&] {

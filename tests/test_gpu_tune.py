@@ -101,3 +101,23 @@ def test_tuning_cache_round_trip(tmp_path):
     strip = lambda cs: [{k: v for k, v in c.items() if k != "ms"} for c in cs]
     assert strip(second) == strip(first)
     assert all(v == 0 for c in second for v in c["ms"].values())
+
+
+@pytest.mark.parametrize("start", ["default", "one chunk per column"])
+def test_autotune_does_not_lose_to_the_starting_schedule(start):
+    """One 64^3 droplet, whose default chunks (2 planes) are no power of two from 8 up and beat those that are: after
+    a tuning, from the default or from a slow schedule, its fused_div and fused_correct take no longer than
+    with the default. 10 % are allowed for the timing."""
+    import ttsh
+
+    def took(s):
+        s.profile_kernels(3)
+        t = [s.profile_kernels(20) for _ in range(6)]
+        return sum(min(p[k][0] for p in t) for k in ("fused_div", "fused_correct"))
+
+    with make(ttsh, (64,), 32) as a:
+        want = took(a)
+        if start != "default":
+            a.set_tuning(0, dict(a.tuning()[0], zc=[64, 64, 64]))
+        a.autotune()
+        assert took(a) <= 1.1 * want, (a.tuning()[0]["zc"], took(a), want)

@@ -804,6 +804,10 @@ void tune_group(ttsh_sim* s, Engine<T>& E, size_t gi, ttsh_tuning* out) {
   }
 }
 
+// Part of a cache entry's key: raised when the kernels or the candidates change, so that entries measured with
+// others are not taken (before the key had a version, the sizes without register kernels had only the
+// Stockham passes to choose from).
+constexpr int kTuneVersion = 2;
 std::string tune_key(const ttsh_sim* s, int N, int n) {
   cudaDeviceProp pr{};
   CK(cudaGetDeviceProperties(&pr, s->device));
@@ -811,8 +815,8 @@ std::string tune_key(const ttsh_sim* s, int N, int n) {
   for (char& c : name)
     if (c == ' ' || c == ':') c = '_';
   char buf[256];
-  std::snprintf(buf, sizeof buf, "%s sm%d%d p%d f%d N%d n%d", name.c_str(), pr.major, pr.minor, s->precision,
-                s->fused ? 1 : 0, N, n);
+  std::snprintf(buf, sizeof buf, "%s sm%d%d v%d p%d f%d N%d n%d", name.c_str(), pr.major, pr.minor, kTuneVersion,
+                s->precision, s->fused ? 1 : 0, N, n);
   return buf;
 }
 

@@ -260,8 +260,8 @@ int ttsh_get_tuning(const ttsh_sim* s, int group, ttsh_tuning* out);
 int ttsh_set_tuning(ttsh_sim* s, int group, const ttsh_tuning* in);
 /* Times the candidates of every group on the instance's own fields and keeps the fastest. The
  * state (phi, P, u, u*, P*, the pressures and T) is left as it was. With cache_path non-NULL,
- * groups with an entry for this GPU, precision, form, N and group size in that text file take
- * it without timing, and the choices of the others are appended to it. */
+ * groups with an entry for this GPU, version of the kernels, precision, form, N and group size in
+ * that text file take it without timing, and the choices of the others are appended to it. */
 int ttsh_autotune(ttsh_sim* s, const char* cache_path);
 
 /* Launch count of one step (kernels of this library). */

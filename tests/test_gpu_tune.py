@@ -121,3 +121,21 @@ def test_autotune_does_not_lose_to_the_starting_schedule(start):
             a.set_tuning(0, dict(a.tuning()[0], zc=[64, 64, 64]))
         a.autotune()
         assert took(a) <= 1.1 * want, (a.tuning()[0]["zc"], took(a), want)
+
+
+def test_cache_entries_of_other_kernels_are_not_taken(tmp_path):
+    """An entry whose key has no version of the kernels, or another one, is left alone: the group is timed and
+    its choice appended."""
+    import re
+    import ttsh
+    cache = tmp_path / "tune.txt"
+    with make(ttsh, (50,), 32) as a:
+        a.autotune(str(cache))
+    key = cache.read_text().split(" : ")[0]
+    for other in (re.sub(r" v\d+", "", key), re.sub(r" v\d+", " v1", key)):
+        old = other + " : 1 1 0 0 0 3 2 5 5\n"  # pinned to the Stockham passes, one line per CTA
+        cache.write_text(old)
+        with make(ttsh, (50,), 32) as a:
+            c = a.autotune(str(cache))[0]
+        assert c["ms"]["fft"] > 0
+        assert cache.read_text().startswith(old + key + " : ")

@@ -993,13 +993,14 @@ static int persistent_grid(const void* kernel, int threads, size_t smem, long lo
 
 // Default schedules of a group of n droplets of size N. fused_rhs: the persistent grid, or, where the group
 // is the batch's only one (alone; the branches of several share the device: 2 x 96^3 .. 192^3 2466 us per
-// step with persistent grids, 2520 with 96^3 in chunks) and one wave of equal chunks has few more planes per CTA than the persistent grid's share, these: a CTA of the
-// persistent grid whose share crosses tiles loads four halo planes again. Measured, us per launch,
-// persistent / chunks (planes per chunk - share): one 96^3 66 / 57 (0.6), one 160^3 219 / 209 (1.4), 2 x 64^3
-// 47 / 43 (1.3), 2 x 96^3 108 / 102 (1.3), 4 x 96^3 192 / 188 (2.5), 3 x 160^3 605 / 593 (2.1), 18 x 64^3 244 /
-// 244 (3.4), 8 x 96^3 355 / 360 (5.1), one 128^3 121 / 131 (5.1); with shares of 1 .. 6 planes the rest of
-// the wave decides (one 64^3, 3.4 planes: 28.5 / 29.3), up to 1 both give every CTA one plane (one 32^3 14.6 /
-// 13.9). fused_div and fused_correct: chunks of z-planes,
+// step with persistent grids, 2520 with 96^3 in chunks) and one wave of equal chunks has at most three more
+// planes per CTA than the persistent grid's share, these: a CTA of the persistent grid whose share crosses
+// tiles loads four halo planes again. Measured, us per launch, persistent / chunks (planes per chunk - share):
+// 3 x 32^3 21.5 / 20.6 (0.7), 8 x 32^3 30.9 / 27.3 (0.6), 14 x 32^3 43.3 / 38.4 (1.1), 20 x 32^3 53.1 / 52.5
+// (2.6), one 64^3 29.2 / 28.3 (0.6), 2 x 64^3 46.7 / 43.0 (1.3), 4 x 64^3 73.3 / 72.3 (2.5), one 96^3 66.3 / 57.8
+// (0.6), 4 x 96^3 192 / 188 (2.5), one 160^3 218 / 209 (1.4), 3 x 160^3 606 / 592 (2.1); beyond the line 18 x 64^3
+// 243.9 / 244.9 (3.4), 30 x 32^3 67.3 / 69.6 (3.4), one 192^3 357 / 360 (5.0), one 128^3 121 / 129 (5.1). Against
+// the rule: one 32^3 14.2 / 14.7 (0.6; its step 32.8 / 30.7). fused_div and fused_correct: chunks of z-planes,
 // long enough to amortise the stencils' two halo planes and the ring's first copies, but short
 // enough that one wave of CTAs covers every SM: the planes are cut into as many chunks as one wave
 // holds (3 or 2 CTAs per SM), at most 40 (fused_div) or 20 (fused_correct) planes each. Measured, us
@@ -1022,7 +1023,7 @@ void fused_default_zc(int N, int n, bool alone, int zc[3]) {
   };
   const int z = planes(2, TYR, N);
   const double places = 2.0 * sms, columns = (double)n * (N / TX) * (N / TYR), share = N * columns / places;
-  zc[0] = alone && columns <= places && z <= share + 3 && (share <= 1 || share >= 6) ? z : 0;
+  zc[0] = alone && columns <= places && z <= share + 3 ? z : 0;
   zc[1] = planes(3, TYD, 40);
   zc[2] = planes(2, TY, 20);
 }

@@ -29,3 +29,16 @@ def test_default_schedule_is_bit_exact(sizes):
     for a, b in zip(*out):
         for f in ("phi", "P", "u", "pv", "pp"):
             assert np.array_equal(a[f], b[f]), f
+
+
+@pytest.mark.parametrize("sizes,chunked", [((32,) * 3, True), ((32,) * 8, True), ((64,), True), ((160,), True), ((128,), False),
+                                           ((64,) * 20, False), ((64, 32), False)])
+def test_fused_rhs_default_follows_the_chunk_length(sizes, chunked):
+    """fused_rhs starts in one wave of chunks wherever these are at most three planes longer than the
+    persistent grid's shares, whatever the share; a batch of several sizes keeps the persistent grid."""
+    import torch
+    import ttsh
+    if torch.cuda.get_device_properties(0).multi_processor_count != 152:
+        pytest.skip("the lengths are those of 152 SMs")
+    with ttsh.Sim([ttsh.default_input(Nx=N, Ny=N, Nz=N) for N in sizes], [ttsh.default_ext(precision=32) for _ in sizes]) as s:
+        assert (s.tuning()[0]["zc"][0] > 0) == chunked, s.tuning()[0]["zc"]

@@ -401,6 +401,7 @@ void build_engine(ttsh_sim* s, Engine<T>& E) {
     G.fft_kind = (fk && std::string(fk) == "stockham") ? 1 : ((fk && std::string(fk) == "separate") ? 0 : 2);
     G.n = (int)E.members[g].size();
     G.N = s->inst[E.members[g][0]].N;
+    CK(cudaDeviceGetAttribute(&G.sms, cudaDevAttrMultiProcessorCount, s->device));
     G.fft_nsteps = E.h[E.members[g][0]].nsteps;
     G.d_err = s->d_err;
     if (s->fused) fused_default_zc(G.N, G.n, E.members.size() == 1, G.zc);

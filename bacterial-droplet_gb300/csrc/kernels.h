@@ -14,6 +14,7 @@ struct Group {
   InstDev<T>* d_inst;  // device array [n]
   int n;               // instances in the group
   int N;
+  int sms = 0;         // SMs of the device (0 where no launch of the group asks)
   int fft_kind = 0;    // register-resident FFT kernels where the size has them, else Stockham: 0 one
                        // launch per axis pass, 2 x and y of a plane in one launch; 1: Stockham only
   int fft_lb = 0;      // Stockham lines per CTA (0: chosen by size, default_lb of fft.cu)

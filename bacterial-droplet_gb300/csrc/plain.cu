@@ -301,7 +301,7 @@ void launch_planes(K kernel, size_t smem, const Group<float>& g, int par, cudaSt
   if ((long)g.N * g.n > 65535) throw std::runtime_error("too many instances of this size in one group");
   const int nx = (g.N + BX - 1) / BX, ny = (g.N + BY - 1) / BY;
   int zc = std::min(16, g.N);
-  while (zc > 1 && (long)nx * ny * g.n * ((g.N + zc - 1) / zc) < 608) zc /= 2;
+  while (zc > 1 && (long)nx * ny * g.n * ((g.N + zc - 1) / zc) < 4 * g.sms) zc /= 2;
   const int nchunk = (g.N + zc - 1) / zc;
   kernel<<<dim3(nx, ny, nchunk * g.n), NT, smem, st>>>(g.d_inst, par, nchunk, zc);
   check_launch(what);
@@ -523,10 +523,10 @@ void launch_correct<float>(const Group<float>& g, int par, cudaStream_t st) {
 }
 template <>
 void launch_stats_u<float>(const Group<float>& g, int, cudaStream_t st) {
-  // planes per CTA: 16 (two halo planes), fewer while the grid is short of a few CTAs per SM
+  // planes per CTA: 16 (two halo planes), fewer while the grid has fewer than eight CTAs per SM
   int zc = std::min(16, g.N);
   const long long tiles = (long long)g.n * ((g.N + BX - 1) / BX) * ((g.N + BY - 1) / BY);
-  while (zc > 2 && tiles * ((g.N + zc - 1) / zc) < 1200) zc /= 2;
+  while (zc > 2 && tiles * ((g.N + zc - 1) / zc) < 8 * g.sms) zc /= 2;
   int nchunk = (g.N + zc - 1) / zc;
   if ((long long)nchunk * g.n > 65535) { nchunk = 1; zc = g.N; }
   k_stats_u<<<dim3((g.N + BX - 1) / BX, (g.N + BY - 1) / BY, nchunk * g.n), BX * BY, 0, st>>>(g.d_inst, nchunk, zc);

@@ -412,6 +412,31 @@ __global__ void __launch_bounds__(STATS_THREADS) k_stats_mass(const InstDev<T>* 
   stats_finish<T>(I, mass, 0.0, 0.0, (double)badn);
 }
 
+// FP32: all diagnostics of a few small droplets in one launch, each thread's share of the mass as in
+// k_stats_mass and then its sites, with the neighbours from global memory: the expressions and bits of
+// k_stats_u, whose launch costs more there than its staged planes save (launch_stats).
+__global__ void __launch_bounds__(STATS_THREADS) k_stats_small(const InstDev<float>* __restrict__ insts, int par) {
+  const InstDev<float>& I = insts[blockIdx.y];
+  const int N = I.N, n = N * N * N;
+  int bad = 0;
+  const double mass = mass_pass<float>(I.phi[par], n, bad);
+  const float c2h = I.ph.c2h;
+  float mdiv = 0.f, mu = 0.f;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    Site s;
+    s.init(i % N, i / N % N, i / (N * N), N);
+    const float d = st_dx<float>(s.acc<float>(I.U[0]), c2h) + st_dy<float>(s.acc<float>(I.U[1]), c2h) + st_dz<float>(s.acc<float>(I.U[2]), c2h);
+    mdiv = fmax(mdiv, fabs(d));
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float u = I.U[a][i], q = I.P[a][i];
+      mu = fmax(mu, fabs(u));
+      if (!isfinite(u) || !isfinite(q)) bad += 1;
+    }
+  }
+  stats_finish<float>(I, mass, (double)mdiv, (double)mu, (double)bad);
+}
+
 // FP32: max |D.u|, max |u| and the non-finite values of u and P, added to the partials of
 // k_stats_mass (maxima and counts do not depend on the order). A CTA sweeps a 32 x 8 column tile over
 // zc planes; the three components' planes (tile + 1) go through a ring of three in shared memory, so
@@ -532,8 +557,25 @@ void launch_stats_u<float>(const Group<float>& g, int, cudaStream_t st) {
   k_stats_u<<<dim3((g.N + BX - 1) / BX, (g.N + BY - 1) / BY, nchunk * g.n), BX * BY, 0, st>>>(g.d_inst, nchunk, zc);
   check_launch("stats (velocity)");
 }
+// FP32, all diagnostics: one launch up to 64^3 while the droplets' STATS_BLOCKS CTAs are one wave (eight per SM).
+// us of a call with its copy to the host, two launches / one: one 8^3 20.3 / 14.5, one 32^3 21.5 / 14.8, one 64^3
+// 24.5 / 24.1, 2 x 40^3 26.7 / 23.7, 3 x 60^3 42.0 / 37.5, 4 x 16^3 34.0 / 29.2, 4 x 54^3 43.9 / 39.6; against the rule
+// 4 x 24^3 33.8 / 35.8, 4 x 60^3 46.1 / 49.1; beyond it one 72^3 26.3 / 27.5, 4 x 80^3 61.5 / 63.4, 8 x 32^3 49.7 / 60.1,
+// 16 x 16^3 78 / 98.
+inline bool stats_in_one(const Group<float>& g) { return g.N <= 64 && (long)g.n * STATS_BLOCKS <= 8L * g.sms; }
+inline bool stats_in_one(const Group<double>&) { return false; }
+inline void launch_stats_small(const Group<float>& g, int par, cudaStream_t st) {
+  k_stats_small<<<dim3(STATS_BLOCKS, g.n), STATS_THREADS, 0, st>>>(g.d_inst, par);
+  check_launch("stats");
+}
+inline void launch_stats_small(const Group<double>&, int, cudaStream_t) {}
+
 template <class T>
 int launch_stats(const Group<T>& g, int par, cudaStream_t st, bool full) {
+  if (full && stats_in_one(g)) {
+    launch_stats_small(g, par, st);
+    return STATS_BLOCKS;
+  }
   k_stats_mass<T><<<dim3(STATS_BLOCKS, g.n), STATS_THREADS, 0, st>>>(g.d_inst, par);
   check_launch("stats");
   if (full) launch_stats_u<T>(g, par, st);

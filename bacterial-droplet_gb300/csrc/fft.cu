@@ -259,6 +259,80 @@ __global__ void __launch_bounds__(FFT_THREADS, fft_min_ctas<T>()) k_fft(const In
   fft_group<T, XAXIS>(insts[blockIdx.y], pass, blockIdx.x, LB, reinterpret_cast<typename CxT<T>::type*>(smem_raw), half);
 }
 
+// FP32, a grid of few CTAs (in_smem): a line group is copied to shared memory, each stage of the plan goes from
+// one buffer to the other, and the result is copied back. A step of fft_group has a thread for every two
+// stages, 20 values at N = 20, and the code of 13 stage pairs is fetched from cold caches; here every stage has a
+// thread for each of its butterflies. The same stages in the same order, so the same bits.
+template <int R, bool INV>
+__device__ __forceinline__ void smem_stage(const float2* src, float2* dst, int N, int LB, int Ns, const float2* tw) {
+  const int M = N / R, pitch = N + 1, ts = N / (Ns * R);
+  for (int b = threadIdx.x; b < LB * M; b += blockDim.x) {
+    const int l = b / M, j = b - l * M, k = j % Ns;
+    float2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = src[l * pitch + j + r * M];
+    plan_butterfly<INV, R>(v, tw, N, k, ts);
+    float2* d = dst + l * pitch + (j / Ns) * Ns * R + k;
+#pragma unroll
+    for (int r = 0; r < R; ++r) d[r * Ns] = v[r];
+  }
+}
+template <bool INV>
+__device__ __forceinline__ void smem_fft(float2*& a, float2*& b, const InstDev<float>& I, int LB) {
+  int Ns = 1;
+  for (int s = 0; s < I.nstages; ++s) {
+    const int R = I.radix[s];
+    if (R == 4) smem_stage<4, INV>(a, b, I.N, LB, Ns, I.tw);
+    else if (R == 2) smem_stage<2, INV>(a, b, I.N, LB, Ns, I.tw);
+    else if (R == 3) smem_stage<3, INV>(a, b, I.N, LB, Ns, I.tw);
+    else smem_stage<5, INV>(a, b, I.N, LB, Ns, I.tw);
+    __syncthreads();
+    float2* t = a;
+    a = b;
+    b = t;
+    Ns *= R;
+  }
+}
+template <int PASS>
+__global__ void __launch_bounds__(FFT_THREADS) k_fft_smem(const InstDev<float>* __restrict__ insts, int LB) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr bool XAXIS = PASS == 0 || PASS == 4;
+  const InstDev<float>& I = insts[blockIdx.y];
+  const int N = I.N, NN = N * N, pitch = N + 1;
+  float2 *a = reinterpret_cast<float2*>(smem_raw), *b = a + LB * pitch;
+  // this group's lines: x rows one after another, or y or z lines adjacent in x
+  const int ng = N / LB, outer = XAXIS ? 0 : blockIdx.x / ng, x0 = XAXIS ? 0 : (blockIdx.x - outer * ng) * LB;
+  float2* const w = I.W + (XAXIS ? blockIdx.x * LB * N : (PASS == 2 ? outer * N : outer * NN) + x0);
+  const int stride = PASS == 2 ? NN : N;
+  // the forward passes, first: both parts of the packed source brought to the same size (pow2_norm)
+  const float su = PASS == 0 && I.wmax ? pow2_norm(I.wmax[0]) : 1.f, sp = PASS == 0 && I.wmax ? pow2_norm(I.wmax[1]) : 1.f;
+  for (int t = threadIdx.x; t < LB * N; t += blockDim.x) {
+    const int e = XAXIS ? t % N : t / LB, l = XAXIS ? t / N : t % LB;
+    float2 v = w[XAXIS ? t : e * stride + l];
+    if (PASS == 0) { v.x *= su; v.y *= sp; }
+    if (PASS >= 3) v.y = -v.y;
+    a[l * pitch + e] = v;
+  }
+  __syncthreads();
+  smem_fft<(PASS >= 3)>(a, b, I, LB);
+  if constexpr (PASS == 2) {
+    for (int t = threadIdx.x; t < LB * N; t += blockDim.x) {
+      const int l = t / N, e = t - l * N;
+      const fftreg::Poisson<float> pm(I, x0 + l, outer);
+      a[l * pitch + e] = dft::conj(pm(a[l * pitch + e], I, e));
+    }
+    __syncthreads();
+    smem_fft<true>(a, b, I, LB);
+  }
+  for (int t = threadIdx.x; t < LB * N; t += blockDim.x) {
+    const int e = XAXIS ? t % N : t / LB, l = XAXIS ? t / N : t % LB;
+    float2 o = a[l * pitch + e];
+    if (PASS >= 2) o.y = -o.y;
+    if (PASS == 4) o = scale_n3(o, I);
+    w[XAXIS ? t : e * stride + l] = o;
+  }
+}
+
 // Both in-plane axes of a z-plane, one thread-block cluster per plane: dir 0 forward x then forward
 // y, dir 1 inverse y then inverse x. As in fftreg_impl.cuh: each CTA of the cluster takes every
 // clusterDim-th line group of the first axis, the cluster barrier (release / acquire) makes the
@@ -343,8 +417,35 @@ inline void check_fft(const char* what) {
   if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+// Lines per CTA of k_fft_smem for this group, 0 where it is not used: boxes up to 64^3 whose grid of
+// power-of-two line groups (the explicit choices, else the largest) has at most five CTAs per SM. FFT of a step
+// (five launches), us, k_fft / this: one 8^3 37.9 / 32.6, one 20^3 60.1 / 36.3, 4 x 20^3 60.7 / 37.0, 16 x 12^3 45.6 /
+// 36.1, one 32^3 48.7 / 41.0, one 48^3 55.5 / 43.0, one 64^3 60.7 / 48.0; against the rule 4 x 18^3 43.9 / 49.0; beyond it
+// 4 x 64^3 81 / 87, one 72^3 55 / 71, 16 x 24^3 47 / 55, 4 x 36^3 53 / 63.
+int smem_lines(const Group<float>& g) {
+  const int lb = g.fft_lb ? fft_lines(g) : pow2_lb(g.N, sizeof(float2));
+  return g.N <= 64 && (long)g.N * (g.N / lb) * g.n <= 5L * g.sms ? lb : 0;
+}
+template <class T>
+bool launch_smem(const Group<T>&, int, cudaStream_t) { return false; }
+template <>
+bool launch_smem<float>(const Group<float>& g, int pass, cudaStream_t st) {
+  const int lb = smem_lines(g);
+  if (!lb) return false;
+  const size_t smem = 2 * (size_t)lb * (g.N + 1) * sizeof(float2);
+  const dim3 grid(g.N * (g.N / lb), g.n);
+  switch (pass) {
+#define X(P) case P: k_fft_smem<P><<<grid, FFT_THREADS, smem, st>>>(g.d_inst, lb); break;
+    X(0) X(1) X(2) X(3) X(4)
+#undef X
+  }
+  check_fft("fft launch");
+  return true;
+}
+
 template <class T>
 void launch_one(const Group<T>& g, int pass, cudaStream_t st) {
+  if (launch_smem<T>(g, pass, st)) return;
   const int N = g.N, LB = fft_lines(g), half = half_values(N, LB);
   const size_t smem = smem_of(g, LB, pass);
   const dim3 grid((N / LB) * N, g.n);

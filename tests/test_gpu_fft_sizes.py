@@ -75,3 +75,25 @@ def test_per_size_kernels_equal_the_any_size_kernel(precision):
                 out.append(s.get_state(0))
         for f in ("pv", "pp", "u", "P"):
             assert np.array_equal(out[0][f], out[1][f]), (N, f)
+
+
+@pytest.mark.parametrize("N,n", [(8, 100), (18, 5), (25, 2), (27, 2), (48, 6), (64, 3)])
+def test_few_and_many_line_groups_give_the_same_bits(N, n):
+    """FP32, one launch per axis: a single droplet's few line groups go through shared memory stage by stage, those of a
+    batch of n as every size's; with the default lines per CTA, one line, and the reverse plan."""
+    import ttsh
+    st = random_state(N, seed=N)
+
+    def run(n, cfg):
+        with ttsh.Sim([ttsh.default_input(Nx=N, Ny=N, Nz=N)] * n, [ttsh.default_ext(precision=32, zeta=0.02, form=ttsh.FORM_PLAIN)] * n) as s:
+            t = s.tuning()[0]
+            s.set_tuning(0, dict(t, fft_kind=1, **({"radix": t["radix"][::-1]} if cfg == "reverse" else {"fft_lb": cfg})))
+            for k in range(n):
+                s.set_state(k, st["phi"], st["P"], st["u"], st["us"], st["ps"])
+            s.step(2)
+            return s.get_state(n - 1)
+
+    for cfg in (0, 1, "reverse"):
+        a, b = run(1, cfg), run(n, cfg)
+        for f in ("phi", "P", "u", "pv", "pp"):
+            assert np.array_equal(a[f], b[f]), (cfg, f)

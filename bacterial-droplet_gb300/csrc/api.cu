@@ -67,11 +67,11 @@ const char* kNames[K_NCLASS] = {"stage1", "stage2", "div", "fft_x_fwd", "fft_y_f
                                 "fft_x_inv", "correct", "fused_rhs", "fused_div", "fused_correct",
                                 "fft_xy_fwd", "fft_yx_inv"};
 
-// The Poisson solve of a group: x+y per plane, z, y+x per plane (fft_kind 2), else one launch per
+// The Poisson solve of a group: x+y per plane, z, y+x per plane (fft_by_plane), else one launch per
 // axis pass. `run(class, launch)` wraps each launch.
 template <class T, class R>
 void enqueue_fft(const Group<T>& g, cudaStream_t st, R&& run) {
-  if (g.fft_kind == 2) {
+  if (fft_by_plane<T>(g)) {
     run(K_FFT_XY, [&] { launch_fft_plane<T>(g, 0, st); });
     run(K_FFT2, [&] { launch_fft_pass<T>(g, 2, st); });
     run(K_FFT_YX, [&] { launch_fft_plane<T>(g, 1, st); });
@@ -80,7 +80,7 @@ void enqueue_fft(const Group<T>& g, cudaStream_t st, R&& run) {
   }
 }
 template <class T>
-int fft_launches(const Group<T>& g) { return g.fft_kind == 2 ? 3 : 5; }
+int fft_launches(const Group<T>& g) { return fft_by_plane<T>(g) ? 3 : 5; }
 
 struct Prof {
   cudaStream_t st;

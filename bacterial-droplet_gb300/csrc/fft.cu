@@ -468,6 +468,17 @@ void fft_steps(int N, const std::vector<int>& plan, int* step, int* nsteps) {
   for (size_t k = 0; k < s.size(); ++k) step[k] = s[k];
 }
 
+// fft_kind 2: by plane at the sizes of the register kernels (which have their own lines and plan) and with the
+// default lines per CTA and, in FP32, the default plan. An explicit choice goes per axis: a plane's cluster has
+// at most eight CTAs, too few for the short lines of the small choices. A step, us, by plane / per axis: FP32 one
+// 25^3 with one line 123 / 47, one 50^3 with two 129 / 94, 16 x 60^3 with four 952 / 881, one 20^3 with the reverse plan
+// 47 / 35; FP64 one 30^3 with two lines 138 / 91; against the rule FP64 16 x 12^3 with four 0.97. In FP64 the reverse
+// plan is as fast by plane (one 50^3 0.98).
+template <class T>
+bool fft_by_plane(const Group<T>& g) {
+  return g.fft_kind == 2 && (fftreg_has<T>(g.N) || (g.fft_lb == 0 && (sizeof(T) == 8 || g.fft_default)));
+}
+
 template <class T>
 void launch_fft_plane(const Group<T>& g, int dir, cudaStream_t st) {
   // the per-size kernels come first: in FP64 the small sizes of the register kernels have them too
@@ -566,6 +577,8 @@ template int fft_lines<float>(const Group<float>&);
 template int fft_lines<double>(const Group<double>&);
 template void launch_fft_pass<float>(const Group<float>&, int, cudaStream_t);
 template void launch_fft_pass<double>(const Group<double>&, int, cudaStream_t);
+template bool fft_by_plane<float>(const Group<float>&);
+template bool fft_by_plane<double>(const Group<double>&);
 template void launch_fft_plane<float>(const Group<float>&, int, cudaStream_t);
 template void launch_fft_plane<double>(const Group<double>&, int, cudaStream_t);
 template void fft_prepare<float>(int);

@@ -63,6 +63,8 @@ template <> void launch_stats_u<double>(const Group<double>&, int, cudaStream_t)
 // Poisson solve by FFT (fft.cu): W <- (inverse FFT of -FFT(W)/k^2) / N^3.
 // pass 0: forward x; 1: forward y; 2: forward z, divide, inverse z; 3: inverse y; 4: inverse x + scale.
 template <class T> void launch_fft_pass(const Group<T>& g, int pass, cudaStream_t st);
+// Whether the group's x and y passes are one launch per plane (launch_fft_plane) or one per axis.
+template <class T> bool fft_by_plane(const Group<T>& g);
 // Forward x + y (dir 0) or inverse y + x (dir 1) of every z-plane in one launch (fft_kind 2): the
 // register kernel of the size, else the one for any size.
 template <class T> void launch_fft_plane(const Group<T>& g, int dir, cudaStream_t st);

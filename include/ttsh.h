@@ -240,7 +240,8 @@ typedef struct {
   int N;           /* droplet size of the group */
   int n;           /* droplets in the group */
   int fft_kind;    /* register-resident kernels where the size has them, else the Stockham ones: 0 one
-                      launch per axis pass, 2 x and y of each plane in one launch; 1 Stockham per axis */
+                      launch per axis pass, 2 x and y of each plane in one launch (per axis where an
+                      explicit fft_lb or, in FP32, another plan is to be run); 1 Stockham per axis */
   int fft_lb;      /* Stockham lines per CTA; 0 = chosen by the size */
   int nstages;     /* Stockham radix plan: radix[0..nstages-1], each 2, 3, 4 or 5, product N */
   int radix[16];

@@ -97,3 +97,20 @@ def test_few_and_many_line_groups_give_the_same_bits(N, n):
         a, b = run(1, cfg), run(n, cfg)
         for f in ("phi", "P", "u", "pv", "pp"):
             assert np.array_equal(a[f], b[f]), (cfg, f)
+
+
+@pytest.mark.parametrize("precision,N,cfg,launches", [(32, 50, {}, 7), (32, 50, {"fft_lb": 2}, 9), (32, 50, {"radix": [5, 5, 2]}, 9),
+                                                      (64, 50, {}, 7), (64, 50, {"fft_lb": 2}, 9), (64, 50, {"radix": [5, 5, 2]}, 7),
+                                                      (32, 64, {"fft_lb": 2}, 7), (64, 64, {"fft_lb": 2}, 7)])
+def test_explicit_choices_go_per_axis(precision, N, cfg, launches):
+    """fft_kind 2: an explicit choice of lines (and in FP32 of the plan) is run one launch per axis at the sizes without
+    register kernels, the defaults by plane; the same bits."""
+    import ttsh
+    inp, ext = ttsh.default_input(Nx=N, Ny=N, Nz=N), ttsh.default_ext(precision=precision, form=ttsh.FORM_PLAIN)
+    with ttsh.Sim(inp, ext) as s:
+        s.set_tuning(0, dict(s.tuning()[0], **cfg))
+        assert s.launches_per_step() == launches
+    if "radix" not in cfg:
+        got, want = projection(N, precision, 2, cfg)[0], projection(N, precision, 2)[0]
+        for f in ("phi", "P", "u", "pv", "pp"):
+            assert np.array_equal(got[f], want[f]), f

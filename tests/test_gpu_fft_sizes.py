@@ -114,3 +114,74 @@ def test_explicit_choices_go_per_axis(precision, N, cfg, launches):
         got, want = projection(N, precision, 2, cfg)[0], projection(N, precision, 2)[0]
         for f in ("phi", "P", "u", "pv", "pp"):
             assert np.array_equal(got[f], want[f]), f
+
+
+# ---- large boxes: one step from white noise, made on the GPU and handed over in page-locked arrays ----
+LARGE = 576  # the largest box below
+
+
+@pytest.fixture(scope="module")
+def noise():
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(1)
+    host = torch.empty(4 * LARGE ** 3, dtype=torch.float64, pin_memory=True)
+    for part in host.split(LARGE ** 3):
+        part.copy_(torch.rand(part.numel(), generator=g, device="cuda", dtype=torch.float64).sub_(0.5).mul_(0.02))
+    torch.cuda.empty_cache()
+    return host.numpy()
+
+
+def solve(noise, N, precision, cfg, provisional=False):
+    """Pressures (and u*, P*) of one step."""
+    import torch
+    import ttsh
+    n = N ** 3
+    pinned = lambda *shape: torch.empty(shape, dtype=torch.float64, pin_memory=True).numpy()
+    with ttsh.Sim(ttsh.default_input(Nx=N, Ny=N, Nz=N), ttsh.default_ext(precision=precision, quirks=0, form=ttsh.FORM_PLAIN)) as s:
+        s.set_tuning(0, dict(s.tuning()[0], **cfg))
+        s.set_state(0, noise[:n].reshape(N, N, N), noise[n:].reshape(-1)[:3 * n].reshape(3, N, N, N), noise[:3 * n].reshape(3, N, N, N))
+        s.step(1)
+        out = [pinned(N, N, N), pinned(N, N, N)]
+        ttsh._check(ttsh.lib().ttsh_get_state(s.handle, 0, None, None, None, ttsh._p(out[0]), ttsh._p(out[1])))
+        if provisional:
+            out += [pinned(3, N, N, N), pinned(3, N, N, N)]
+            ttsh._check(ttsh.lib().ttsh_get_provisional(s.handle, 0, ttsh._p(out[2]), ttsh._p(out[3])))
+        return out
+
+
+def against_cufft(out, tol):
+    import torch
+    import ttsh
+    inp = ttsh.default_input()
+    for got, want in zip(out, cufft_projection(out[2], out[3], inp.h, inp.dt0)):
+        assert relerr(got, want) <= tol, relerr(got, want)
+    torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("N", [n for n in range(271, 501) if all(p in (2, 3, 5) for p in _factors(n))])
+def test_large_per_size_kernels_equal_the_any_size_kernel(noise, N, precision):
+    """The sizes above 270 with kernels of their own: the bits of the kernel for any size."""
+    for a, b in zip(*(solve(noise, N, precision, {"fft_kind": kind}) for kind in (2, 1))):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision,tol", [(64, 1e-12), (32, 2e-5)])
+@pytest.mark.parametrize("N", [540, 576])
+def test_any_size_kernel_above_500(noise, N, precision, tol):
+    """Sizes without kernels of their own: the plane launches with the default lines per CTA against cuFFT, one launch
+    per axis and one line per CTA the same bits."""
+    want = solve(noise, N, precision, {}, True)
+    against_cufft(want, tol)
+    for cfg in ({"fft_kind": 1}, {"fft_lb": 1}):
+        for a, b in zip(solve(noise, N, precision, cfg), want):
+            assert np.array_equal(a, b), cfg
+
+
+@pytest.mark.parametrize("N", [64, 96, 128, 160, 192, 256, 512])
+def test_fp64_register_kernels_match_cufft(noise, N):
+    """The FP64 register kernels, x and y of a plane in one launch, against cuFFT; per axis the same bits."""
+    want = solve(noise, N, 64, {}, True)
+    against_cufft(want, 1e-12)
+    for a, b in zip(solve(noise, N, 64, {"fft_kind": 0}), want):
+        assert np.array_equal(a, b)

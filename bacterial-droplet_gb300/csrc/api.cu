@@ -286,20 +286,17 @@ void build_engine(ttsh_sim* s, Engine<T>& E) {
     for (int i : E.members[kv.second]) {
       const double h = s->inst[i].in.h;
       if (tab.count({N, h})) continue;
-      std::vector<double> kval(N);
       std::vector<T> t3(3 * N);  // k^2, sin(k h)/h, (2 + cos(k h))/3
       for (int k = 0; k < N; ++k) {
         // initPoissonSolver (TTSH3D.cu:1093-1117)
         double kk = 2 * kPi * k / (N * h + 0.0);
         if (k >= N / 2) kk = 2 * kPi * (k - N) / (N * h + 0.0);
-        kval[k] = kk;
         t3[k] = (T)(kk * kk);
         t3[N + k] = (T)(std::sin(kk * h) / h);
         t3[2 * N + k] = (T)((2.0 + std::cos(kk * h)) / 3.0);
       }
       InstDev<T> t{};
       t.tw = d_tw;
-      t.kval = static_cast<const double*>(upload(kval.data(), N * sizeof(double)));
       t.k2t = static_cast<const T*>(upload(t3.data(), 3 * N * sizeof(T)));
       t.St = t.k2t + N;
       t.Ct = t.St + N;

@@ -71,8 +71,7 @@ struct InstDev {
   T* mu[3];
   T* sig[9];          // sig[a*3+b] = phi * D_a P_b
   const C* tw;        // tw[k] = exp(-2 pi i k / N), k < N
-  const double* kval; // k(m), FP64 (continuous wavenumber of initPoissonSolver)
-  const T* k2t;       // k(m)^2 rounded to T
+  const T* k2t;       // k(m)^2 rounded to T, k(m) the continuous wavenumber of initPoissonSolver
   const T* St;        // sin(k h)/h
   const T* Ct;        // (2 + cos(k h))/3
   double* red;        // FP64 reduction partials
@@ -133,84 +132,26 @@ __device__ __forceinline__ void stats_add(const InstDev<T>& I, int k, long long 
   if (bad) atomicAdd(out + 3, (double)bad);
 }
 
-// Accessor of a scalar field around (x,y,z) with periodic wrap.
+// Accessor of a scalar field in global memory around (x,y,z) with periodic wrap.
 template <class T>
 struct Acc {
   const T* __restrict__ f;
   int xo[3], yo[3], zo[3];
-  int stride;  // 1 for real arrays, 2 for one component of an interleaved complex array
-  __device__ __forceinline__ T operator()(int dx, int dy, int dz) const {
-    return __ldg(f + (size_t)stride * (zo[dz + 1] + yo[dy + 1] + xo[dx + 1]));
-  }
-};
-
-// Accessor whose wrapped neighbours come from `old` (quirk Q2 of the reference:
-// the halo of u*/P* is refreshed at the start of getRHS, TTSH3D.cu:369-371 and
-// :405-407, before getVStar rewrites the interior, :471-491).
-template <class T>
-struct AccStale {
-  const T* __restrict__ f;
-  const T* __restrict__ old;
-  int xo[3], yo[3], zo[3];
-  bool wx[3], wy[3], wz[3];
-  __device__ __forceinline__ T operator()(int dx, int dy, int dz) const {
-    const T* p = (wx[dx + 1] | wy[dy + 1] | wz[dz + 1]) ? old : f;
-    return __ldg(p + zo[dz + 1] + yo[dy + 1] + xo[dx + 1]);
-  }
-};
-
-// Accessor of the pointwise product phi * Pa * Pb (build-defined active stress).
-template <class T>
-struct AccProd {
-  const T* __restrict__ phi;
-  const T* __restrict__ pa;
-  const T* __restrict__ pb;
-  int xo[3], yo[3], zo[3];
-  __device__ __forceinline__ T operator()(int dx, int dy, int dz) const {
-    int i = zo[dz + 1] + yo[dy + 1] + xo[dx + 1];
-    return __ldg(phi + i) * __ldg(pa + i) * __ldg(pb + i);
-  }
+  __device__ __forceinline__ T operator()(int dx, int dy, int dz) const { return __ldg(f + (zo[dz + 1] + yo[dy + 1] + xo[dx + 1])); }
 };
 
 struct Site {
   int xo[3], yo[3], zo[3];
-  bool wx[3], wy[3], wz[3];
-  int idx;
   __device__ __forceinline__ void init(int x, int y, int z, int N) {
     int NN = N * N;
     xo[0] = wrapi(x - 1, N); xo[1] = x; xo[2] = wrapi(x + 1, N);
     yo[0] = wrapi(y - 1, N) * N; yo[1] = y * N; yo[2] = wrapi(y + 1, N) * N;
     zo[0] = wrapi(z - 1, N) * NN; zo[1] = z * NN; zo[2] = wrapi(z + 1, N) * NN;
-    wx[0] = x == 0; wx[1] = false; wx[2] = x == N - 1;
-    wy[0] = y == 0; wy[1] = false; wy[2] = y == N - 1;
-    wz[0] = z == 0; wz[1] = false; wz[2] = z == N - 1;
-    idx = z * NN + y * N + x;
   }
   template <class T>
-  __device__ __forceinline__ Acc<T> acc(const T* f, int stride = 1) const {
+  __device__ __forceinline__ Acc<T> acc(const T* f) const {
     Acc<T> a;
     a.f = f;
-    a.stride = stride;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) { a.xo[i] = xo[i]; a.yo[i] = yo[i]; a.zo[i] = zo[i]; }
-    return a;
-  }
-  template <class T>
-  __device__ __forceinline__ AccStale<T> acc_stale(const T* f, const T* old) const {
-    AccStale<T> a;
-    a.f = f;
-    a.old = old;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      a.xo[i] = xo[i]; a.yo[i] = yo[i]; a.zo[i] = zo[i];
-      a.wx[i] = wx[i]; a.wy[i] = wy[i]; a.wz[i] = wz[i];
-    }
-    return a;
-  }
-  template <class T>
-  __device__ __forceinline__ AccProd<T> acc_prod(const T* phi, const T* pa, const T* pb) const {
-    AccProd<T> a;
-    a.phi = phi; a.pa = pa; a.pb = pb;
 #pragma unroll
     for (int i = 0; i < 3; ++i) { a.xo[i] = xo[i]; a.yo[i] = yo[i]; a.zo[i] = zo[i]; }
     return a;

@@ -15,17 +15,12 @@
 namespace ttsh {
 namespace fftreg {
 
-template <class C>
-__device__ __forceinline__ C cmul(C a, C b) {
-  C r;
+__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
+  float2 r;
   r.x = a.x * b.x - a.y * b.y;
   r.y = a.x * b.y + a.y * b.x;
   return r;
 }
-template <class C>
-__device__ __forceinline__ C cadd(C a, C b) { C r; r.x = a.x + b.x; r.y = a.y + b.y; return r; }
-template <class C>
-__device__ __forceinline__ C csub(C a, C b) { C r; r.x = a.x - b.x; r.y = a.y - b.y; return r; }
 // FP32: one packed instruction (add/sub .f32x2: two IEEE FP32 operations, round to nearest, the
 // results of the two scalar ones) per complex add or subtract.
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
@@ -51,24 +46,20 @@ constexpr int first_radix(int L) { return L % 4 == 0 ? 4 : (L % 2 == 0 ? 2 : (L 
 template <class C, int NF>
 __device__ C ctw(int k);
 
-// twiddle k of the DFT's table: the __constant__ copy when the line length NF is known (NF > 0),
-// else the table in global memory
-template <class C, bool INV, int NF>
-__device__ __forceinline__ C twx(const C* t, int k) {
-  if constexpr (NF > 0) {
-    C w = ctw<C, NF>(k);
-    if (INV) w.y = -w.y;
-    return w;
-  } else {
-    return tw<C, INV>(t, k);
-  }
+// ... conjugate for the inverse
+template <bool INV, int NF>
+__device__ __forceinline__ float2 twx(int k) {
+  float2 w = ctw<float2, NF>(k);
+  if (INV) w.y = -w.y;
+  return w;
 }
 
-// In-place DFT of v[0..L) (natural order in and out). `step` = N / L, so that w_L^m = tab[m*step].
-// NF: the table's length when it has a __constant__ copy (0: read `tab`).
-template <class C, int L, bool INV, int NF = 0>
+// FP32: in-place DFT of v[0..L) (natural order in and out), a factor of a line of length NF. `step` = NF / L, so
+// that w_L^m is entry m step of the line's table.
+template <int L, bool INV, int NF>
 struct Dft {
-  static __device__ __forceinline__ void run(C* v, const C* tab, int step) {
+  typedef float2 C;
+  static __device__ __forceinline__ void run(C* v, int step) {
     constexpr int R = first_radix(L);
     constexpr int M = L / R;
     if constexpr (L == 1) {
@@ -91,7 +82,7 @@ struct Dft {
       for (int q = 0; q < L; ++q) {
         C acc = v[0];
 #pragma unroll
-        for (int r = 1; r < L; ++r) acc = cadd(acc, cmul(v[r], twx<C, INV, NF>(tab, ((q * r) % L) * step)));
+        for (int r = 1; r < L; ++r) acc = cadd(acc, cmul(v[r], twx<INV, NF>(((q * r) % L) * step)));
         o[q] = acc;
       }
 #pragma unroll
@@ -103,14 +94,14 @@ struct Dft {
       for (int r = 0; r < R; ++r) {
 #pragma unroll
         for (int m = 0; m < M; ++m) u[r][m] = v[r + R * m];
-        Dft<C, M, INV, NF>::run(u[r], tab, step * R);
+        Dft<M, INV, NF>::run(u[r], step * R);
       }
 #pragma unroll
       for (int k0 = 0; k0 < M; ++k0) {
         C t[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) t[r] = (r > 0 && k0 > 0) ? cmul(u[r][k0], twx<C, INV, NF>(tab, r * k0 * step)) : u[r][k0];
-        Dft<C, R, INV, NF>::run(t, tab, step * M);
+        for (int r = 0; r < R; ++r) t[r] = (r > 0 && k0 > 0) ? cmul(u[r][k0], twx<INV, NF>(r * k0 * step)) : u[r][k0];
+        Dft<R, INV, NF>::run(t, step * M);
 #pragma unroll
         for (int k1 = 0; k1 < R; ++k1) v[k0 + M * k1] = t[k1];
       }

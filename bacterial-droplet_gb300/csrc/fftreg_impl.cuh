@@ -104,15 +104,14 @@ __device__ __forceinline__ C tw4(const C* tab, int k) {
   }
 }
 
-// PASS: 0 forward x, 1 forward y, 2 forward z + Poisson multiplier + inverse z, 3 inverse y,
+// FP32. PASS: 0 forward x, 1 forward y, 2 forward z + Poisson multiplier + inverse z, 3 inverse y,
 // 4 inverse x scaled by 1/N^3. One call transforms line group g of the pass (LB lines) with the
 // CTA's threads; S is the CTA's shared memory. SIN (z pass only): the group's input is already in
 // shared memory, In[z * LB + line]; `after` runs once every thread has read it (In may then be
 // refilled).
-template <class T, int N1, int N2, int PASS, bool SIN = false, class F = NoOp>
-__device__ __forceinline__ void fft_lines(const InstDev<T>& I, int g, typename CxT<T>::type* S,
-                                          const typename CxT<T>::type* In = nullptr, F after = F()) {
-  typedef typename CxT<T>::type C;
+template <int N1, int N2, int PASS, bool SIN = false, class F = NoOp>
+__device__ __forceinline__ void fft_lines32(const InstDev<float>& I, int g, float2* S, const float2* In = nullptr, F after = F()) {
+  typedef float2 C;
   constexpr int N = N1 * N2;
   constexpr int LB = lines_per_cta<N>();
   constexpr int OW = N1 / N2;  // k1 rows owned by each thread in the second step
@@ -153,32 +152,32 @@ __device__ __forceinline__ void fft_lines(const InstDev<T>& I, int g, typename C
 #pragma unroll
       for (int n1 = 0; n1 < N1; ++n1) v[n1] = W[base + (size_t)(N2 * n1 + j) * stride];
     }
-    if constexpr (PASS == 0 && sizeof(T) == 4) {
-      // FP32: both parts of the packed source brought to the same size (pow2_norm, common.cuh)
+    if constexpr (PASS == 0) {
+      // both parts of the packed source brought to the same size (pow2_norm, common.cuh)
       if (I.wmax) {
-        const T su = pow2_norm(I.wmax[0]), sp = pow2_norm(I.wmax[1]);
+        const float su = pow2_norm(I.wmax[0]), sp = pow2_norm(I.wmax[1]);
 #pragma unroll
         for (int n1 = 0; n1 < N1; ++n1) { v[n1].x *= su; v[n1].y *= sp; }
       }
     }
-    Dft<C, N1, false, N>::run(v, tab, N2);
+    Dft<N1, false, N>::run(v, N2);
 #pragma unroll
     for (int k1 = 0; k1 < N1; ++k1) S[sidx(k1, j)] = (k1 > 0 && j > 0) ? cmul(v[k1], tw4<C, false, N, TW4C>(tab, j * k1)) : v[k1];
     __syncthreads();
     after();
-    const Poisson<T> pm(I, xl, yl);  // used by the z pass
+    const Poisson<float> pm(I, xl, yl);  // used by the z pass
 #pragma unroll
     for (int o = 0; o < OW; ++o) {
       const int k1 = j + N2 * o;
       C u[N2];
 #pragma unroll
       for (int n2 = 0; n2 < N2; ++n2) u[n2] = S[sidx(k1, n2)];
-      Dft<C, N2, false, N>::run(u, tab, N1);
+      Dft<N2, false, N>::run(u, N1);
       if constexpr (PASS == 2) {
         // spectrum element z = k1 + N1*k2 of the line (x = xl, y = yl): multiply, go back
 #pragma unroll
         for (int k2 = 0; k2 < N2; ++k2) u[k2] = pm(u[k2], I, k1 + N1 * k2);
-        Dft<C, N2, true, N>::run(u, tab, N1);
+        Dft<N2, true, N>::run(u, N1);
 #pragma unroll
         for (int n2 = 0; n2 < N2; ++n2) S[sidx(k1, n2)] = (n2 > 0 && k1 > 0) ? cmul(u[n2], tw4<C, true, N, TW4C>(tab, n2 * k1)) : u[n2];
       } else {
@@ -191,7 +190,7 @@ __device__ __forceinline__ void fft_lines(const InstDev<T>& I, int g, typename C
       C x[N1];
 #pragma unroll
       for (int k1 = 0; k1 < N1; ++k1) x[k1] = S[sidx(k1, j)];
-      Dft<C, N1, true, N>::run(x, tab, N2);
+      Dft<N1, true, N>::run(x, N2);
 #pragma unroll
       for (int n1 = 0; n1 < N1; ++n1) W[base + (size_t)(N2 * n1 + j) * stride] = x[n1];
     }
@@ -203,7 +202,7 @@ __device__ __forceinline__ void fft_lines(const InstDev<T>& I, int g, typename C
       C u[N2];
 #pragma unroll
       for (int k2 = 0; k2 < N2; ++k2) u[k2] = W[base + (size_t)(k1 + N1 * k2) * stride];
-      Dft<C, N2, true, N>::run(u, tab, N1);
+      Dft<N2, true, N>::run(u, N1);
 #pragma unroll
       for (int n2 = 0; n2 < N2; ++n2) S[sidx(k1, n2)] = (n2 > 0 && k1 > 0) ? cmul(u[n2], tw4<C, true, N, TW4C>(tab, n2 * k1)) : u[n2];
     }
@@ -211,7 +210,7 @@ __device__ __forceinline__ void fft_lines(const InstDev<T>& I, int g, typename C
     C x[N1];
 #pragma unroll
     for (int k1 = 0; k1 < N1; ++k1) x[k1] = S[sidx(k1, j)];
-    Dft<C, N1, true, N>::run(x, tab, N2);
+    Dft<N1, true, N>::run(x, N2);
 #pragma unroll
     for (int n1 = 0; n1 < N1; ++n1) {
       C v = x[n1];
@@ -309,7 +308,7 @@ __device__ __forceinline__ void fft_lines64(const InstDev<double>& I, int g, dou
 template <class T, int N1, int N2, int PASS>
 __device__ __forceinline__ void fft_group(const InstDev<T>& I, int g, typename CxT<T>::type* S) {
   if constexpr (sizeof(T) == 8) fft_lines64<N1, N2, PASS>(I, g, S);
-  else fft_lines<T, N1, N2, PASS>(I, g, S);
+  else fft_lines32<N1, N2, PASS>(I, g, S);
 }
 
 // Minimum CTAs per SM. The FP32 z pass (forward, divide, inverse) is bound by latency and issue and
@@ -513,7 +512,7 @@ __global__ void __launch_bounds__(lines_per_cta<N1 * N2>() * N2, zt_min_blocks<N
     ok = __syncthreads_and(mbar_wait_bounded(&bar[s], (unsigned)(k / ZST) & 1u, limit)) != 0;
     if (!ok) break;
     const int inst = g / NG, gn = g + ZST * gridDim.x;
-    fft_lines<float, N1, N2, 2, true>(insts[inst], g - inst * NG, S, In + (size_t)s * N * LB, [&] {
+    fft_lines32<N1, N2, 2, true>(insts[inst], g - inst * NG, S, In + (size_t)s * N * LB, [&] {
       if (tid == 0 && gn < total) {
         issue(gn, s);
         issued[s] = k + ZST;

@@ -68,18 +68,18 @@ bool g_prepared[256][kMaxN + 1] = {{false}};
 int fail(int code, const std::string& msg) { return ttsh::set_error(code, "ttsh_step_noalloc: " + msg); }
 
 // What one call writes into the tail of the working array before its steps: the droplet
-// descriptor, the twiddles exp(-2 pi i k / N) and the wavenumber tables (k, k^2, sin(k h)/h,
+// descriptor, the twiddles exp(-2 pi i k / N) and the wavenumber tables (k^2, sin(k h)/h,
 // (2 + cos(k h))/3), passed by value as a kernel parameter (about 2 KB, within the 4 KB limit).
 struct Setup {
   ttsh::InstDev<double> inst;
   double2 tw[kMaxN];
-  double tab[4 * kMaxN];
+  double tab[3 * kMaxN];
 };
 static_assert(sizeof(Setup) <= 4000, "set-up parameter within the kernel parameter limit");
 
 __global__ void k_noalloc_setup(const Setup s, ttsh::InstDev<double>* d_inst, double2* d_tw, double* d_tab) {
   for (int i = threadIdx.x; i < kMaxN; i += blockDim.x) d_tw[i] = s.tw[i];
-  for (int i = threadIdx.x; i < 4 * kMaxN; i += blockDim.x) d_tab[i] = s.tab[i];
+  for (int i = threadIdx.x; i < 3 * kMaxN; i += blockDim.x) d_tab[i] = s.tab[i];
   if (threadIdx.x == 0) *d_inst = s.inst;
 }
 
@@ -180,8 +180,7 @@ extern "C" int ttsh_step_noalloc(const ttsh_input* in, const ttsh_ext* ext, int 
     I.W = reinterpret_cast<double2*>(take(2 * n));
     unsigned char* tail = base + kFieldsBytes;
     double2* d_tw = reinterpret_cast<double2*>(tail);
-    double* d_kval = reinterpret_cast<double*>(tail + 8192);
-    double* d_k2t = d_kval + kMaxN;
+    double* d_k2t = reinterpret_cast<double*>(tail + 8192);
     double* d_St = d_k2t + kMaxN;
     double* d_Ct = d_St + kMaxN;
     InstDev<double>* d_inst = reinterpret_cast<InstDev<double>*>(tail + 32768);
@@ -193,10 +192,9 @@ extern "C" int ttsh_step_noalloc(const ttsh_input* in, const ttsh_ext* ext, int 
       su.tw[k] = make_double2(std::cos(a), std::sin(a));
       double kk = 2 * kPi * k / (N * h + 0.0);
       if (k >= N / 2) kk = 2 * kPi * (k - N) / (N * h + 0.0);
-      su.tab[k] = kk;
-      su.tab[kMaxN + k] = kk * kk;
-      su.tab[2 * kMaxN + k] = std::sin(kk * h) / h;
-      su.tab[3 * kMaxN + k] = (2.0 + std::cos(kk * h)) / 3.0;
+      su.tab[k] = kk * kk;
+      su.tab[kMaxN + k] = std::sin(kk * h) / h;
+      su.tab[2 * kMaxN + k] = (2.0 + std::cos(kk * h)) / 3.0;
     }
     I.N = N;
     I.stale = (ext->quirks & TTSH_QUIRK_STALE_HALO) ? 1 : 0;
@@ -223,7 +221,7 @@ extern "C" int ttsh_step_noalloc(const ttsh_input* in, const ttsh_ext* ext, int 
       I.Us[0][b] = ustar + b * n; I.Us[1][b] = us_new + b * n;
       I.Ps[0][b] = Pstar + b * n; I.Ps[1][b] = ps_new + b * n;
     }
-    I.tw = d_tw; I.kval = d_kval; I.k2t = d_k2t; I.St = d_St; I.Ct = d_Ct;
+    I.tw = d_tw; I.k2t = d_k2t; I.St = d_St; I.Ct = d_Ct;
     I.red = nullptr;
 #define NA_CK(call)                                                                 \
   do {                                                                              \
@@ -231,7 +229,7 @@ extern "C" int ttsh_step_noalloc(const ttsh_input* in, const ttsh_ext* ext, int 
     if (e_ != cudaSuccess) throw std::runtime_error(std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
     // descriptor and tables into the working array, in stream order, by value (no host copy)
-    k_noalloc_setup<<<1, 128, 0, st>>>(su, d_inst, d_tw, d_kval);
+    k_noalloc_setup<<<1, 128, 0, st>>>(su, d_inst, d_tw, d_k2t);
     NA_CK(cudaGetLastError());
     Group<double> g{d_inst, 1, N};
     g.fft_kind = 2;

@@ -303,8 +303,7 @@ void build_engine(ttsh_sim* s, Engine<T>& E) {
       tab[{N, h}] = t;
     }
     fft_prepare<T>(N);
-    if (sizeof(T) == 8) plain64_prepare(N);
-    else if (!s->fused) plain32_prepare();
+    if (sizeof(T) == 4 && !s->fused) plain32_prepare();
     if (fftreg_has<T>(N)) fftreg_twiddles<T>(N);
   }
   // per-instance arenas

@@ -42,8 +42,6 @@ template <class T> void launch_div(const Group<T>& g, int par, cudaStream_t st);
 template <class T> void launch_correct(const Group<T>& g, int par, cudaStream_t st);
 // Sets the FP32 kernels' dynamic shared-memory limits (call before capture).
 void plain32_prepare();
-// Sets the FP64 kernels' dynamic shared-memory limits for size N (call before capture).
-void plain64_prepare(int N);
 template <> void launch_stage1<float>(const Group<float>&, int, cudaStream_t);
 template <> void launch_stage2<float>(const Group<float>&, int, cudaStream_t);
 template <> void launch_div<float>(const Group<float>&, int, cudaStream_t);

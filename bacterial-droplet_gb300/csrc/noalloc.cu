@@ -156,7 +156,6 @@ extern "C" int ttsh_step_noalloc(const ttsh_input* in, const ttsh_ext* ext, int 
       std::lock_guard<std::mutex> lk(g_mu);
       if (!g_prepared[dev][N]) {
         fft_prepare<double>(N);
-        plain64_prepare(N);
         if (fftreg_has<double>(N)) fftreg_twiddles<double>(N);  // the register FFT's constant table
         // the table copy runs on the legacy stream: let it land before kernels on any stream read it
         const cudaError_t es = cudaDeviceSynchronize();

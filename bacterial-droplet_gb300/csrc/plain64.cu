@@ -10,10 +10,10 @@
 #include <cstdio>
 #include <stdexcept>
 #include <string>
-#include <utility>
 
 #include "common.cuh"
 #include "kernels.h"
+#include "tiles.h"
 
 namespace ttsh {
 
@@ -46,44 +46,7 @@ inline void check_launch(const char* what) {
 typedef double T;
 typedef double2 C;
 typedef InstDev<double> Inst;
-constexpr int MAXT = 256;  // threads (sites of a tile) at most
 constexpr int CTAS = 3;    // CTAs per SM that registers and shared memory leave room for
-
-struct TileDim {
-  int tx, ty, nx, ny;  // columns, rows; tiles per row and column of a plane
-  int threads() const { return (tx * ty + 31) / 32 * 32; }
-};
-
-// The tile of size N: rows of the box in nx equal parts, columns in ny, such that the FP64
-// instructions per plane, counted in whole warps (3 per point of pass z, 6 of pass x, 25 of pass y
-// and the pointwise terms), are fewest: 32 x 8 at N = 64 and 256, 25 x 10 at N = 100 (32-column tiles
-// would leave 22 % of the lanes outside the box), 24 x 8 at N = 48.
-TileDim pick_tile(int N) {
-  static thread_local int last_n = 0;
-  static thread_local TileDim last;
-  if (last_n == N) return last;
-  TileDim best{};
-  long cost = 0;
-  for (int nx = 1; nx <= N; ++nx) {
-    const int tx = (N + nx - 1) / nx;
-    if (tx > 64) continue;
-    if (tx < 8 && tx < N) break;
-    for (int ny = 1; ny <= N; ++ny) {
-      const int ty = (N + ny - 1) / ny;
-      if (tx * ty > MAXT) continue;
-      if (ty < 4 && ty < N) break;
-      auto warps = [](int points) { return (points + 31) / 32; };
-      const long c = (long)nx * ny * (3 * warps((tx + 2) * (ty + 2)) + 6 * warps(tx * (ty + 2)) + 25 * warps(tx * ty));
-      if (!best.tx || c < cost) {
-        best = TileDim{tx, ty, nx, ny};
-        cost = c;
-      }
-    }
-  }
-  last_n = N;
-  last = best;
-  return best;
-}
 
 // What a thread knows of its CTA's tile. Staged points of pass z are the (tx + 2) x (ty + 2) of the
 // tile and its halo (row-major), of pass x the tx x (ty + 2).
@@ -152,8 +115,6 @@ template <int NF>
 struct GradLap {
   T *v, *c, *s, *d;     // pass z: the value, c_z, s_z, delta_z
   T *xd, *xs, *xz, *xc; // pass x: delta_x s_z, s_x s_z, s_x delta_z, c_x c_z
-  static __host__ __device__ size_t values(int np, int nx) { return (size_t)NF * 4 * (np + nx); }
-
   __device__ __forceinline__ GradLap(T* m, int np, int nx) {
     v = m;
     c = v + NF * np;
@@ -540,44 +501,20 @@ __global__ void __launch_bounds__(MAXT, CTAS) k_stats_u(const Inst* __restrict__
   if ((threadIdx.x & 31) == 0) stats_add(I, blockIdx.x + gridDim.x * (blockIdx.z % N), mdiv, mu, bad);
 }
 
-// Shared-memory values (of T) of each kernel for a tile.
-inline size_t stage1_values(const TileDim& d) { return GradLap<2>::values((d.tx + 2) * (d.ty + 2), d.tx * (d.ty + 2)); }
-inline size_t stage2_values(const TileDim& d) {
-  const size_t np = (size_t)(d.tx + 2) * (d.ty + 2), nx = (size_t)d.tx * (d.ty + 2);
-  return 9 * np + 6 * nx;  // the divergences; the Laplacians take 8 np + 4 nx
-}
-inline size_t div_values(const TileDim& d) { return 6 * (size_t)(d.tx + 2) * (d.ty + 2) + 2 * (size_t)d.tx * (d.ty + 2); }
-inline size_t stats_values(const TileDim& d) { return 3 * (size_t)(d.tx + 2) * (d.ty + 2) + (size_t)d.tx * (d.ty + 2); }
-inline size_t correct_values(const TileDim& d) {
-  return 4 * (size_t)(d.tx + 2) * (d.ty + 2) + 4 * (size_t)d.tx * (d.ty + 2);
-}
-
 template <class K>
 void launch_tiles(K kernel, const Group<double>& g, int par, size_t (*values)(const TileDim&), cudaStream_t st, const char* what) {
   if ((long)g.N * g.n > 65535) throw std::runtime_error("too many instances of this size in one group");
-  const TileDim d = pick_tile(g.N);
+  static thread_local TileDim d;
+  static thread_local int last_n = 0;
+  if (last_n != g.N) {
+    d = pick_tile(g.N);
+    last_n = g.N;
+  }
   kernel<<<dim3(d.nx * d.ny, 1, g.N * g.n), d.threads(), values(d) * sizeof(T), st>>>(g.d_inst, par, d.tx, d.ty, d.nx);
   check_launch(what);
 }
 
 }  // namespace
-
-void plain64_prepare(int N) {
-  const TileDim d = pick_tile(N);
-  const std::pair<const void*, size_t> k[] = {{(const void*)k_stage1, stage1_values(d)},
-                                              {(const void*)k_stage2, stage2_values(d)},
-                                              {(const void*)k_div, div_values(d)},
-                                              {(const void*)k_correct, correct_values(d)},
-                                              {(const void*)k_stats_u, stats_values(d)}};
-  // one kernel serves every size: its limit is only ever raised
-  for (const auto& f : k) {
-    cudaFuncAttributes fa{};
-    cudaError_t e = cudaFuncGetAttributes(&fa, f.first);
-    if (e == cudaSuccess && (size_t)fa.maxDynamicSharedSizeBytes < f.second * sizeof(T))
-      e = cudaFuncSetAttribute(f.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(f.second * sizeof(T)));
-    if (e != cudaSuccess) throw std::runtime_error(std::string("plain kernels' smem attribute: ") + cudaGetErrorString(e));
-  }
-}
 
 template <>
 void launch_stage1<double>(const Group<double>& g, int par, cudaStream_t st) {

@@ -22,7 +22,7 @@ struct Phys {
   T c2h;           // 1/(2h)
   T cl12, cl23, cl143;  // 1/(12h^2), 2/(3h^2), 14/(3h^2)
   T clz;           // 1/h^2 (the fused form's shift-invariant Laplacian)
-  T invN3;         // 1/N^3 (FP32 path); FP64 path divides by (double)N^3 as getStream mode 2
+  T invN3;         // 1/N^3, the factor of getStream mode 2
   // constants of the FP64 form's separable stencils, whose sums have integer weights: 1/(72 h) of D,
   // the same over dt, and 1/(12 h^2) of L times kPhi, La^2, mu, gamma, eta
   T kd, kdiv, kPhi12, La212, mu12, gamma12, eta12;
@@ -69,7 +69,7 @@ struct InstDev {
   int* smax;                       // max |u*|, max |P*| of this step (float bits): the divergence's grid
   T* mu0;             // plain-form intermediates
   T* mu[3];
-  T* sig[9];          // sig[a*3+b] = phi * D_a P_b
+  T* sig[9];          // sig[a*3+b]: FP32 phi D_a P_b, FP64 cA phi D_a P_b - zeta phi P_a P_b
   const C* tw;        // tw[k] = exp(-2 pi i k / N), k < N
   const T* k2t;       // k(m)^2 rounded to T, k(m) the continuous wavenumber of initPoissonSolver
   const T* St;        // sin(k h)/h

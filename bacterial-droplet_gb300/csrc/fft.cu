@@ -15,13 +15,14 @@
 //   3 inverse y   4 inverse x, scaled by 1/N^3 (getStream mode 2, :684-690)
 // The inverse transform is the forward one between conjugations.
 //   FP64 (bound by the FP64 pipe): steps of radix 2 .. 16 with the small DFTs of dft.cuh, chosen by
-//     size (N = 100 is 10 x 10, N = 320 is 8 x 8 x 5); a radix-5 butterfly is 36 operations instead of
+//     size (N = 100 is 10 x 10, N = 320 is 10 x 8 x 4); a radix-5 butterfly is 36 operations instead of
 //     the 120 of the sum that defines it. Pass 2 multiplies by -1/k^2 and begins the inverse in the
 //     registers of the forward transform's last step, whose outputs (elements j + r N/R) are the
 //     inputs of a first step of the same radix.
 //   FP32 (bound by latency and issue): the stages of the radix plan (4, 2, 3, 5), up to two of them
 //     in registers per step: the butterflies of one stage feed those of the next within a thread, so
-//     the arithmetic is the plan's, stage by stage, with half the trips through shared memory.
+//     the arithmetic is the plan's, stage by stage, with half the trips through shared memory. Few line
+//     groups, one launch per axis: one stage per step (k_fft_smem).
 // Twiddles between steps come from a table exp(-2 pi i k/N) built on the host in FP64.
 #include <algorithm>
 #include <cstdio>

@@ -5,7 +5,8 @@
 //   X[k1 + N1*k2] = DFT_N2 over n2 of w_N^(n2*k1) * Y[k1][n2]    (after one shared-memory transpose)
 // and the inverse runs the same steps backwards. Each thread keeps its N1 (or N2) values in
 // registers; small DFTs are expanded at compile time by mixed-radix decimation in time
-// (radix 4, 2, and the 3- and 5-point ones of dft.cuh), with twiddles read from the FP64-built table exp(-2 pi i k / N).
+// (FP32: radix 4, 2, and 3 and 5 as the sums that define them; FP64: dft.cuh), with twiddles from the FP64-built table
+// exp(-2 pi i k / N).
 // The z pass goes forward, applies the Poisson multiplier and goes back without leaving the
 // CTA: two shared-memory transposes for the whole forward-divide-inverse sequence.
 #pragma once

@@ -42,7 +42,7 @@ inline void check_launch(const char* what) {
 // L = cl12 (c_x c_y c_z + 8 faces - 56 centre) are the reference's 27-point and 15-point weights
 // (st_dx/st_dy/st_dz/st_lap of common.cuh, TTSH3D.cu:3280-3343): the weights are integers until one
 // last multiplication, where the reference rounds 16/36, 4/36 and 1/36. A gradient and a Laplacian
-// of one field take about 25 operations per site of a 32 x 8 tile instead of about 90.
+// of one field take about 24 operations per site of a 16 x 16 tile instead of about 90.
 typedef double T;
 typedef double2 C;
 typedef InstDev<double> Inst;
@@ -176,7 +176,7 @@ struct GradLap {
 // which stage 2 differentiates, and the rates of change that need no second derivative, which go to
 // the output arrays u*, P*, phi' for stage 2 to complete. About 245 FP64 operations per site;
 // forming the products on chip, as the fused FP32 form does, would repeat them on every tile's halo
-// (1.33 times at 32 x 8), while the 20 words per site written and read back here take a tenth of
+// (1.27 times at 16 x 16), while the 20 words per site written and read back here take a tenth of
 // the time of the arithmetic.
 __global__ void __launch_bounds__(MAXT, CTAS) k_stage1(const Inst* __restrict__ insts, int par, int tx, int ty, int ntx) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(MAXT, CTAS) k_stage1(const Inst* __restrict__ 
   const Phys<T>& p = I.ph;
   T* const sm = reinterpret_cast<T*>(smem_raw);
   const int o = t.o;
-  // two fields at a time, so that three CTAs fit on an SM (43 KB each): with four at a time and two
+  // two fields at a time, so that three CTAs fit on an SM (39 KB each at 16 x 16): with four at a time and two
   // CTAs the FP64 pipe idled 18 % of the time at the barriers between the passes
   T P[3] = {0, 0, 0}, u[3] = {0, 0, 0}, w[3] = {0, 0, 0}, gp[3] = {0, 0, 0};  // w = u + lambda0 P
   T ph = 0, mu0 = 0, kap = 0, m = 0;

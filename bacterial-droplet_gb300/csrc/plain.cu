@@ -557,12 +557,11 @@ void launch_stats_u<float>(const Group<float>& g, int, cudaStream_t st) {
   k_stats_u<<<dim3((g.N + BX - 1) / BX, (g.N + BY - 1) / BY, nchunk * g.n), BX * BY, 0, st>>>(g.d_inst, nchunk, zc);
   check_launch("stats (velocity)");
 }
-// FP32, all diagnostics: one launch up to 64^3 while the droplets' STATS_BLOCKS CTAs are one wave (eight per SM).
-// us of a call with its copy to the host, two launches / one: one 8^3 20.3 / 14.5, one 32^3 21.5 / 14.8, one 64^3
-// 24.5 / 24.1, 2 x 40^3 26.7 / 23.7, 3 x 60^3 42.0 / 37.5, 4 x 16^3 34.0 / 29.2, 4 x 54^3 43.9 / 39.6; against the rule
-// 4 x 24^3 33.8 / 35.8, 4 x 60^3 46.1 / 49.1; beyond it one 72^3 26.3 / 27.5, 4 x 80^3 61.5 / 63.4, 8 x 32^3 49.7 / 60.1,
-// 16 x 16^3 78 / 98.
-inline bool stats_in_one(const Group<float>& g) { return g.N <= 64 && (long)g.n * STATS_BLOCKS <= 8L * g.sms; }
+// FP32, all diagnostics: one launch up to 64^3 and three droplets (STATS_BLOCKS CTAs each, at most six per SM). us of
+// a call with its copy to the host, two launches / one: one 8^3 20.3 / 14.5, one 32^3 21.5 / 14.8, one 64^3 24.5 /
+// 24.1, 2 x 40^3 26.7 / 23.7, 3 x 24^3 31.7 / 29.2 (35.4 in some runs), 3 x 60^3 42.0 / 37.5; beyond the rule one 72^3 26.3 /
+// 27.5, 4 x 16^3 34.0 / 29.2 .. 35.5, 4 x 24^3 33.8 / 35.8, 4 x 54^3 43.9 / 39.6 .. 48.2, 8 x 32^3 49.7 / 60.1, 16 x 16^3 78 / 98.
+inline bool stats_in_one(const Group<float>& g) { return g.N <= 64 && (long)g.n * STATS_BLOCKS <= 6L * g.sms; }
 inline bool stats_in_one(const Group<double>&) { return false; }
 inline void launch_stats_small(const Group<float>& g, int par, cudaStream_t st) {
   k_stats_small<<<dim3(STATS_BLOCKS, g.n), STATS_THREADS, 0, st>>>(g.d_inst, par);

@@ -59,7 +59,7 @@ def test_nonfinite_is_counted(precision, field, value):
 
 @pytest.mark.parametrize("N", [8, 18, 27, 64])
 def test_one_and_two_launches_give_the_same_bits(N):
-    """FP32: one to four small droplets take one launch, more of them two; the same diagnostics for the same state."""
+    """FP32: up to three small droplets take one launch, more of them two; the same diagnostics for the same state."""
     import ttsh
     st = [random_state(N, seed=N + k) for k in range(2)]
 
@@ -70,7 +70,7 @@ def test_one_and_two_launches_give_the_same_bits(N):
             return s.reduce_all()
 
     many = stats(24)
-    for n in (1, 4):
+    for n in (1, 3, 4):
         for a, b in zip(stats(n), many):
             assert a == b
 
